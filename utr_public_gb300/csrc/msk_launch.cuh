@@ -296,9 +296,10 @@ struct Launch {
                          cudaStream_t s)
     {
         static std::once_flag f;
-        set_smem(k_row_expv<N>, Smem<N>::row, f);
-        const int L = RowCfg<N>::L;
-        k_row_expv<N><<<nunits * row_blocks(g, L), L * P::T, Smem<N>::row, s>>>(g, v, ustride, out);
+        constexpr int L = RowCfg<N>::LT;
+        constexpr size_t sm = (size_t)L * P::PADN * 8;
+        set_smem(k_row_expv<N>, sm, f);
+        k_row_expv<N><<<nunits * row_blocks(g, L), L * P::T, sm, s>>>(g, v, ustride, out);
     }
     static void row_adj_transmit(const Geom &g, int nunits, float2 *Gu, float2 *B,
                                  const float2 *Wp, cudaStream_t s)

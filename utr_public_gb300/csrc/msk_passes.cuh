@@ -137,8 +137,8 @@ __device__ __forceinline__ float scat_dI(float2 phi)
 // Rows (lines of length NY) per CTA for the row passes.
 template <int NY> struct RowCfg {
     static constexpr int T = FftPlan<NY>::T;
-    static constexpr int L = (256 / T) > 0 ? 256 / T : 1;   // P1 and the row utilities
-    static constexpr int LT = (128 / T) > 0 ? 128 / T : 1;  // P3 (two tiles in flight)
+    static constexpr int L = (256 / T) > 0 ? 256 / T : 1;   // P1 and most row utilities
+    static constexpr int LT = (128 / T) > 0 ? 128 / T : 1;  // the adjoint transmit, k_row_expv
     static constexpr bool BLK = T > 32;
     // resident CTAs per SM the latency-bound utilities are compiled for
     // (80 registers a thread at 256 threads); fewer where that would spill
@@ -820,13 +820,15 @@ k_row_intensity(const Geom g, const int *__restrict__ img_off, const int *__rest
 // Rows of a per-slice potential stack v[u][k][ix][iy] (float, V*Angstrom):
 // A = S(exp(i sigma v) - 1), the scattered part tau of the transmission
 // before its band limit.  `v` points at slice k of unit 0; units are
-// `ustride` floats apart.
+// `ustride` floats apart.  CTAs of 128 threads, five per SM: the 96 registers
+// hold the line as pairs (at 80, the share of three 256-thread CTAs, 260 bytes a
+// thread spill: 3.7 ms of a 16-unit 512^2 adjoint against 2.9; 3.1 before).
 template <int NY>
-__global__ void __launch_bounds__(RowCfg<NY>::L * FftPlan<NY>::T, RowCfg<NY>::MB)
+__global__ void __launch_bounds__(RowCfg<NY>::LT * FftPlan<NY>::T, NY <= 1024 ? 5 : 4)
 k_row_expv(const Geom g, const float *__restrict__ v, size_t ustride, float2 *__restrict__ out)
 {
     using P = FftPlan<NY>;
-    constexpr int T = P::T, E = P::E, L = RowCfg<NY>::L;
+    constexpr int T = P::T, E = P::E, L = RowCfg<NY>::LT;
     constexpr bool BLK = RowCfg<NY>::BLK;
     extern __shared__ __align__(128) unsigned char smem[];
     float2 *s_lines = reinterpret_cast<float2 *>(smem);
