@@ -393,4 +393,103 @@ __device__ __forceinline__ void fft_line(float2 (&v)[FftPlan<N, EV>::E], float2 
     }
 }
 
+// Point m of the E that a thread of a line of N points holds in strided order
+// (index t + m T, t < T = N/E) lies beyond the 2/3 band limit for every t: the
+// band keeps |k| < N/3.
+template <int E> __host__ __device__ constexpr bool band_zero(int m)
+{
+    return 3 * m > E && 3 * (m + 1) <= 2 * E;
+}
+
+// A thread's stage twiddles held in registers, for kernels that transform many
+// lines per thread: loaded once (at 1024 points 31 of them, 62 registers)
+// instead of 16 table loads per transform.
+template <int N, int R, int NS, int EV = 0>
+struct StageRegs {
+    static constexpr int T = FftPlan<N, EV>::T, KB = FftPlan<N, EV>::E / R;
+    static constexpr int KD = T % NS == 0 ? 1 : KB;  // sub-transforms with twiddles of their own
+    float2 w[KD * (R > 1 ? R - 1 : 1)];
+    __device__ __forceinline__ void load(const float2 *tw, int t)
+    {
+        const float4 *tw4 = reinterpret_cast<const float4 *>(tw);
+#pragma unroll
+        for (int k = 0; k < KD; k++) {
+            const int j = (t + k * T) % NS;
+#pragma unroll
+            for (int p = 0; p < R / 2; p++) {
+                const float4 q = __ldg(&tw4[p * NS + j]);
+                w[k * (R - 1) + 2 * p] = make_float2(q.x, q.y);
+                if (2 * p + 2 < R) w[k * (R - 1) + 2 * p + 1] = make_float2(q.z, q.w);
+            }
+        }
+    }
+    __device__ __forceinline__ float2 get(int k, int r) const { return w[(k % KD) * (R - 1) + r - 1]; }
+};
+template <int N, int EV = 0>
+struct LineRegs {
+    using P = FftPlan<N, EV>;
+    StageRegs<N, P::R2, P::NS2, EV> s2;
+    StageRegs<N, P::R3, P::NS3, EV> s3;
+    __device__ __forceinline__ void load(const float2 *tw, int t)
+    {
+        if constexpr (P::S >= 2) s2.load(tw, t);
+        if constexpr (P::S == 3) s3.load(tw + P::TW2, t);
+    }
+};
+
+// ---------------------------------------------------------------- one line in steps
+// The two-stage transform of one line (64 to 1024 points, 32 a thread) as its
+// steps, for kernels that do something between them; twiddles in registers.
+//   line_first: the first stage and its result into the exchange buffer, with
+//               a warp barrier before and after (ZIN as for fft_pair)
+//   line_read:  the exchanged line out of the buffer
+//   line_last:  twiddles and the last stage
+template <int N, bool INV, bool ZIN>
+__device__ __forceinline__ void line_first(float2 (&v)[32], float2 *buf, int t)
+{
+    static_assert(FftPlan<N>::S == 2 && FftPlan<N>::T <= 32, "one warp, two stages");
+    float2 a[32];
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+        float2 &s = a[brev(i, 5)], &d = a[brev(i, 5) + 1];
+        const float2 p = v[i], q = v[i + 16];
+        if (ZIN && band_zero<32>(i + 16)) {
+            s = d = p;
+        } else if (ZIN && band_zero<32>(i)) {
+            s = q;
+            d = make_float2(-q.x, -q.y);
+        } else {
+            s = cadd(p, q);
+            d = csub(p, q);
+        }
+    }
+    dft_levels<32, INV, 1, 4>(a);
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < 32; r++) buf[pidx<N>(t * 32 + r)] = a[r];
+    __syncwarp();
+}
+template <int N>
+__device__ __forceinline__ void line_read(float2 (&v)[32], const float2 *buf, int t)
+{
+    using P = FftPlan<N>;
+    constexpr int R = P::R2, KB = 32 / R;
+#pragma unroll
+    for (int k = 0; k < KB; k++)
+#pragma unroll
+        for (int r = 0; r < R; r++) v[k + r * KB] = buf[pidx<N>(t + k * P::T + r * (N / R))];
+}
+template <int N, bool INV>
+__device__ __forceinline__ void line_last(float2 (&v)[32], const LineRegs<N> &tw)
+{
+    constexpr int R = FftPlan<N>::R2, KB = 32 / R;
+#pragma unroll
+    for (int k = 0; k < KB; k++) {
+#pragma unroll
+        for (int r = 1; r < R; r++)
+            v[k + r * KB] = INV ? cmul_conj(v[k + r * KB], tw.s2.get(k, r)) : cmul(v[k + r * KB], tw.s2.get(k, r));
+        dft<R, INV, KB>(&v[k]);
+    }
+}
+
 }  // namespace msk

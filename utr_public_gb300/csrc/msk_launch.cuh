@@ -18,6 +18,19 @@ struct ColView {
     int v;
 };
 
+// SMs of the current device.
+inline int sm_count()
+{
+    static std::mutex m;
+    static int known[64];
+    int d = 0, n = 0;
+    if (cudaGetDevice(&d) != cudaSuccess || d < 0 || d >= 64) return 1;
+    std::lock_guard<std::mutex> lk(m);
+    if (known[d]) return known[d];
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, d) != cudaSuccess || n < 1) return 1;
+    return known[d] = n;
+}
+
 struct SizeOps {
     int n;
     int col_c[kColVariants], col_box_rows;  // column tile widths per variant, TMA box height
@@ -237,6 +250,37 @@ struct Launch {
         k_row_transmit<N, SCAT, EV, W><<<nunits * row_blocks(g, L), L * TrCfg<N, EV, W>::T, sm, s>>>(
             g, units, tbuf, psi, out, out_scale, band);
     }
+    // The streamed form of the 32-point plan, from five jobs per warp of the GPU:
+    // below that its last round leaves warps idle and its CTAs keep the passes of
+    // the other stream off the SMs.  Slice loops of 1024^2 with every launch
+    // streamed against none: 4 units 3.95 / 3.73 ms, 8 6.84 / 6.75, 10 8.28 /
+    // 8.34, 16 12.5 / 13.0, 48 32.4 / 34.4; 512^2: 24 units 7.12 / 7.00, 48 12.09
+    // / 12.11, 192 40.5 / 42.2.
+    template <bool SCAT>
+    static bool row_stream(const Geom &g, const int *units, int nunits, const float2 *tbuf,
+                           const float2 *psi, float2 *out, float out_scale, int band, cudaStream_t s)
+    {
+        using R = RsCfg<N>;
+        if constexpr (R::OK) {
+            const int sms = sm_count();
+            const long long njobs = (long long)nunits * (g.nx / R::RW);
+            if (g.nx % R::RW || njobs < 5ll * sms * kRsWarps || njobs > 0x7fffffff) return false;
+            static std::once_flag fb, fw;
+            if (band && g.seg_e1 <= R::Z0 && g.seg_s2 >= R::Z1) {
+                set_smem(k_row_stream<N, SCAT, true>, R::SMEM, fb);
+                k_row_stream<N, SCAT, true><<<sms, 32 * kRsWarps, R::SMEM, s>>>(
+                    g, units, tbuf, psi, out, out_scale, (int)njobs);
+            } else if (!band) {
+                set_smem(k_row_stream<N, SCAT, false>, R::SMEM, fw);
+                k_row_stream<N, SCAT, false><<<sms, 32 * kRsWarps, R::SMEM, s>>>(
+                    g, units, tbuf, psi, out, out_scale, (int)njobs);
+            } else {
+                return false;
+            }
+            return true;
+        }
+        return false;
+    }
     template <bool SCAT>
     static void row_transmit_t(const Geom &g, const int *units, int nunits, const float2 *tbuf,
                                const float2 *psi, float2 *out, float out_scale, int band, int rv,
@@ -250,7 +294,7 @@ struct Launch {
         }
         if (rv == 1)
             row_transmit_v<SCAT, 0, 128>(g, units, nunits, tbuf, psi, out, out_scale, band, s);
-        else
+        else if (!row_stream<SCAT>(g, units, nunits, tbuf, psi, out, out_scale, band, s))
             row_transmit_v<SCAT, 0, 64>(g, units, nunits, tbuf, psi, out, out_scale, band, s);
     }
     static void row_init(const Geom &g, const int *units, int nunits, const float2 *wave0,

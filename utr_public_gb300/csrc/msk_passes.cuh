@@ -146,9 +146,10 @@ template <int NY> struct RowCfg {
 };
 // The transmit's schedules, chosen per row length at run time by timing them
 // (the row tuner of the host code): the FFT plan EV and the CTA width W.
-//   variant 0: EV = 0 (32 points a thread), CTAs of 64 threads (rows of up to
-//              32 threads: two or more rows a CTA, so a CTA barrier waits for
-//              fewer warps; the registers of six CTAs per SM)
+//   variant 0: EV = 0 (32 points a thread); launches of enough rows of 64 to
+//              1024 points stream (k_row_stream), the others run in CTAs of 64
+//              threads (rows of up to 32 threads: two or more rows a CTA, so a
+//              CTA barrier waits for fewer warps; the registers of six CTAs per SM)
 //   variant 1: EV = 0, CTAs of 128 threads (three per SM)
 //   variant 2: (64 to 2048 points) EV = 16 (16 points a thread), CTAs of 128
 //              threads, four per SM at 128 registers; a 2048-point row is one
@@ -730,6 +731,219 @@ k_row_transmit(const Geom g, const int *__restrict__ units, const float2 *__rest
         bulk_store(out + off, bufW, bytes);
         bulk_commit();
         bulk_wait_read();
+    }
+}
+
+// The streamed transmit (rows of 64 to 1024 points): one CTA of kRsWarps warps
+// per SM, every warp on its own with a job of 32 / T rows (1024 points) at a
+// time, every 12 x gridDim-th.  Two buffers a warp: X takes the transmission
+// rows, Y the wave rows.  X is free once iS(B) has read its exchange, and the
+// next job's transmission rows load into it there and then; Y once the result
+// has left it, and the next wave rows load while iS(B) of the next job runs: no
+// load is waited for, and no barrier is wider than a warp.  iS(B) waits in
+// tensor memory (64 words a lane) for its product with iS(W), which spares a
+// third buffer (16 KB more a warp would halve the warps) and a pass of it
+// through the shared-memory pipe, the busiest unit here; the twiddles stay in
+// registers.  BAND: in-band row segments move, the inputs beyond them are
+// neither read nor filled and the outputs there not computed.
+// Bound: FMA pipe (55-60%) and issue slots at the 12 warps that 168 registers
+// and two buffers each allow; the row segments alone would take 63 ms of the
+// 180-orientation 1024^2 series, whose transmits take 93.6 ms in this form and
+// 116.6 ms as k_row_transmit (bulk loads waited for by every CTA, zero fills
+// copied into the rows, three unrolled transforms).
+constexpr int kRsWarps = 12;
+template <int NY> struct RsCfg {
+    static constexpr bool OK = NY >= 64 && NY <= 1024;
+    static constexpr int T = FftPlan<NY>::T;
+    static constexpr int RW = T <= 32 ? 32 / T : 1;  // rows a job
+    static constexpr int BUF = RW * FftPlan<NY>::PADN;  // float2 per buffer
+    static constexpr int Z0 = 11 * NY / 32, Z1 = 21 * NY / 32;  // band_zero's points
+    static constexpr size_t SMEM = (size_t)kRsWarps * (2 * BUF * 8 + 16) + 16;
+    static constexpr int TCOLS = 256;  // tensor-memory columns: 64 for each third warp
+};
+
+__device__ __forceinline__ void tmem_put(uint32_t addr, const float2 (&v)[32])
+{
+#define MSK_W(i) "r"(__float_as_uint(v[i].x)), "r"(__float_as_uint(v[i].y))
+#define MSK_W16(o) MSK_W(o), MSK_W(o + 1), MSK_W(o + 2), MSK_W(o + 3), MSK_W(o + 4), MSK_W(o + 5), \
+    MSK_W(o + 6), MSK_W(o + 7), MSK_W(o + 8), MSK_W(o + 9), MSK_W(o + 10), MSK_W(o + 11),          \
+    MSK_W(o + 12), MSK_W(o + 13), MSK_W(o + 14), MSK_W(o + 15)
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+        asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, "
+                     "%10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, "
+                     "%26, %27, %28, %29, %30, %31, %32};" ::"r"(addr + 32 * h), MSK_W16(16 * h)
+                     : "memory");
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+#undef MSK_W16
+#undef MSK_W
+}
+
+// Half h of what tmem_put stored (16 complex values).
+__device__ __forceinline__ void tmem_get(uint32_t addr, int h, float2 (&v)[16])
+{
+#define MSK_R(i) "=f"(v[i].x), "=f"(v[i].y)
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, "
+                 "%10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, "
+                 "%26, %27, %28, %29, %30, %31}, [%32];"
+                 : MSK_R(0), MSK_R(1), MSK_R(2), MSK_R(3), MSK_R(4), MSK_R(5), MSK_R(6), MSK_R(7),
+                   MSK_R(8), MSK_R(9), MSK_R(10), MSK_R(11), MSK_R(12), MSK_R(13), MSK_R(14), MSK_R(15)
+                 : "r"(addr + 32 * h)
+                 : "memory");
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#undef MSK_R
+}
+
+template <int NY, bool SCAT, bool BAND>
+__global__ void __launch_bounds__(32 * kRsWarps, 1)
+k_row_stream(const Geom g, const int *__restrict__ units, const float2 *__restrict__ tbuf,
+             const float2 *psi, float2 *out, float out_scale, int njobs)
+{
+    using R = RsCfg<NY>;
+    constexpr int T = R::T, E = 32, RW = R::RW, PADN = FftPlan<NY>::PADN;
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, l = lane / T, t = lane % T;
+    float2 *bufs = reinterpret_cast<float2 *>(smem) + warp * 2 * R::BUF;  // X, then Y
+    uint64_t *bar = reinterpret_cast<uint64_t *>(reinterpret_cast<float2 *>(smem) +
+                                                 kRsWarps * 2 * R::BUF) + 2 * warp;
+    uint32_t *tmem_base = reinterpret_cast<uint32_t *>(reinterpret_cast<float2 *>(smem) +
+                                                       kRsWarps * (2 * R::BUF + 2));
+    if (warp == 0)
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                         smem_u32(tmem_base)), "n"(R::TCOLS)
+                     : "memory");
+    if (lane == 0) {
+        mbar_init(&bar[0], 1);
+        mbar_init(&bar[1], 1);
+        fence_mbar_init();
+    }
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tm = *tmem_base + ((uint32_t)(warp & 3) << 21) + 64u * (warp >> 2);
+
+    const int jpu = g.nx / RW;  // jobs per unit
+    const int e1 = g.seg_e1, s2 = g.seg_s2;
+    const int first = blockIdx.x * kRsWarps + warp, step = gridDim.x * kRsWarps;
+    auto offset = [&](int job) {  // of the job's first row
+        const int q = job / jpu;
+        return ((size_t)(units ? units[q] : q) * g.nx + (size_t)(job - q * jpu) * RW) * NY;
+    };
+    // the points between the segments and the band_zero ones read as zeros: with
+    // the full 2/3 band they are some of m = 10 and m = 21 (chosen as they are
+    // read), with a narrower one (the other axis limits it) zeros fill them
+    const bool fill = BAND && (e1 < 10 * T || s2 > 22 * T);
+    auto load = [&](int b, const float2 *src, size_t off) {  // by the whole warp: lane r row r
+        if (lane == 0)
+            mbar_arrive_expect_tx(&bar[b], (!BAND ? NY : fill ? R::Z0 + NY - R::Z1 : e1 + NY - s2) * RW * 8);
+        if (BAND) {
+            if (lane < RW) {
+                float2 *d = bufs + b * R::BUF + lane * NY;
+                const float2 *q = src + off + (size_t)lane * NY;
+                if (e1 > 0) bulk_load(d, q, e1 * 8, &bar[b]);
+                if (s2 < NY) bulk_load(d + s2, q + s2, (NY - s2) * 8, &bar[b]);
+                if (fill && e1 < R::Z0) bulk_load(d + e1, g.zeros, (R::Z0 - e1) * 8, &bar[b]);
+                if (fill && s2 > R::Z1) bulk_load(d + R::Z1, g.zeros, (s2 - R::Z1) * 8, &bar[b]);
+            }
+        } else if (lane == 0) {
+            bulk_load(bufs + b * R::BUF, src + off, RW * NY * 8, &bar[b]);
+        }
+    };
+    bool more = first < njobs;
+    size_t off = more ? offset(first) : 0;
+    if (more) {
+        load(0, tbuf, off);
+        load(1, psi, off);
+    }
+    LineRegs<NY> tw;
+    tw.load(g.tw_row, t);
+    uint32_t parity = 0;
+    for (int job = first; more; job += step, parity ^= 1) {
+        const bool next = job + step < njobs;
+        const size_t noff = next ? offset(job + step) : 0;
+        float2 v[E];
+#pragma unroll 1
+        for (int b = 0; b < 2; b++) {  // iS(B), then iS(W): one copy of the transform's code
+            if (!__all_sync(0xffffffffu, mbar_wait(&bar[b], parity))) {
+                // give up, once the warp's other loads in flight have landed (or after a limit)
+                if (lane == 0) atomicOr(g.err, kErrWaitTimeout);
+                (void)mbar_wait(&bar[0], parity);
+                if (b == 1 || job == first) (void)mbar_wait(&bar[1], parity);
+                if (b == 1 && next) (void)mbar_wait(&bar[0], parity ^ 1);
+                more = false;
+                break;
+            }
+            float2 *buf = bufs + b * R::BUF;
+#pragma unroll
+            for (int m = 0; m < E; m++)
+                if (!BAND || !band_zero<E>(m)) v[m] = buf[l * NY + t + m * T];
+            if (BAND && !fill) {
+                if (t + 10 * T >= e1) v[10] = make_float2(0.0f, 0.0f);
+                if (t + 21 * T < s2) v[21] = make_float2(0.0f, 0.0f);
+            }
+            __syncwarp();  // dense rows read before an exchange overwrites them
+            line_first<NY, true, BAND>(v, buf + l * PADN, t);
+            if (b == 0 && job != first) {  // the last result has left Y: its next wave rows
+                bulk_wait_read();
+                __syncwarp();
+                load(1, psi, off);
+            }
+            line_read<NY>(v, buf + l * PADN, t);
+            if (b == 0 && next) {  // X is read: the next transmission rows
+                fence_proxy_async();
+                __syncwarp();
+                load(0, tbuf, noff);
+            }
+            line_last<NY, true>(v, tw);
+            if (b == 0) tmem_put(tm, v);
+        }
+        if (!more) break;
+        float2 *buf = bufs + R::BUF;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            float2 q[16];
+            tmem_get(tm, h, q);
+#pragma unroll
+            for (int m = 0; m < 16; m++)
+                v[16 * h + m] = SCAT ? scat_transmit(v[16 * h + m], q[m], 1.0f / (float)NY)
+                                     : cmul(v[16 * h + m], q[m]);
+        }
+        __syncwarp();  // iS(W)'s exchange is read
+        line_first<NY, false, false>(v, buf + l * PADN, t);
+        line_read<NY>(v, buf + l * PADN, t);
+        line_last<NY, false>(v, tw);
+        __syncwarp();  // the exchange is read: dense rows into its place
+#pragma unroll
+        for (int m = 0; m < E; m++) {
+            if (BAND && band_zero<E>(m)) continue;
+            buf[l * NY + t + m * T] = out_scale == 1.0f ? v[m] : cscale(v[m], out_scale);
+        }
+        fence_proxy_async();
+        __syncwarp();
+        if (BAND) {
+            if (lane < RW) {
+                float2 *d = out + off + (size_t)lane * NY, *q = buf + lane * NY;
+                // the (at most two) out-of-band elements inside the segments
+                if (e1 > 0 && out_of_band(g, e1 - 1)) q[e1 - 1] = make_float2(0.0f, 0.0f);
+                if (s2 < NY && out_of_band(g, s2)) q[s2] = make_float2(0.0f, 0.0f);
+                fence_proxy_async();
+                if (e1 > 0) bulk_store(d, q, e1 * 8);
+                if (s2 < NY) bulk_store(d + s2, q + s2, (NY - s2) * 8);
+            }
+        } else if (lane == 0) {
+            bulk_store(out + off, buf, RW * NY * 8);
+        }
+        bulk_commit();
+        more = next;
+        off = noff;
+    }
+    bulk_wait_read();
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(*tmem_base),
+                     "n"(R::TCOLS));
     }
 }
 
