@@ -1021,25 +1021,38 @@ void prof_collect(msk_context *ctx)
 namespace {
 
 // Times launch(v) for the variants v in [0, nv): two warm-up launches of every
-// variant, then kTuneRounds rounds in which every variant runs once between two
+// variant, then kTuneRounds rounds in which every variant runs between two
 // events, the order rotating from round to round; ms[v] = the variant's fastest
-// launch.  Interleaving the variants keeps a clock that is still rising (the
-// first launches of a process) from favouring whichever variant runs last.
+// run.  Interleaving the variants keeps a clock that is still rising (the
+// first launches of a process) from favouring whichever variant runs last.  A
+// run is as many launches back to back as take about kTuneMs: the event clock
+// moves in steps of 2 us, as much as the variants of a small grid differ by
+// (one launch of 14 us a run chose another plan from process to process).
 template <typename F>
 bool time_variants(cudaStream_t s, int nv, F launch, float *ms)
 {
     constexpr int kTuneRounds = 5;
+    constexpr float kTuneMs = 0.2f;
     std::vector<cudaEvent_t> ev((size_t)2 * nv * kTuneRounds, nullptr);
     bool ok = true;
     for (auto &e : ev) ok = ok && cudaEventCreate(&e) == cudaSuccess;
     for (int w = 0; w < 2 && ok; w++)
         for (int v = 0; v < nv; v++) launch(v);
+    int reps = 1;
+    if (ok) {
+        float t = 0.0f;
+        ok = cudaEventRecord(ev[0], s) == cudaSuccess;
+        for (int i = 0; i < 4; i++) launch(0);
+        ok = ok && cudaEventRecord(ev[1], s) == cudaSuccess && cudaEventSynchronize(ev[1]) == cudaSuccess &&
+             cudaEventElapsedTime(&t, ev[0], ev[1]) == cudaSuccess;
+        if (ok) reps = std::max(1, std::min(32, (int)(kTuneMs / std::max(t / 4.0f, 1e-3f) + 0.5f)));
+    }
     for (int r = 0; r < kTuneRounds && ok; r++)
         for (int i = 0; i < nv && ok; i++) {
             const int v = (i + r) % nv;
             cudaEvent_t *e = &ev[(size_t)2 * (r * nv + v)];
             ok = cudaEventRecord(e[0], s) == cudaSuccess;
-            launch(v);
+            for (int k = 0; k < reps; k++) launch(v);
             ok = ok && cudaEventRecord(e[1], s) == cudaSuccess;
         }
     ok = ok && cudaStreamSynchronize(s) == cudaSuccess && cudaGetLastError() == cudaSuccess;
@@ -1049,7 +1062,7 @@ bool time_variants(cudaStream_t s, int nv, F launch, float *ms)
             float t = 0.0f;
             ok = cudaEventElapsedTime(&t, ev[(size_t)2 * (r * nv + v)],
                                       ev[(size_t)2 * (r * nv + v) + 1]) == cudaSuccess;
-            ms[v] = std::min(ms[v], t);
+            ms[v] = std::min(ms[v], t / (float)reps);
         }
     }
     for (auto &e : ev)
