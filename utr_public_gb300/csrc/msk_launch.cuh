@@ -108,8 +108,8 @@ const SizeOps *size_ops(int n);
 
 template <int N> struct Smem {
     using P = FftPlan<N>;
-    static constexpr int NTS = RowCfg<N>::L * P::T;
-    static constexpr size_t splat = (size_t)RowCfg<N>::L * SplatCfg<N>::SROW * 8 + NTS * 16 +
+    static constexpr int NTS = SplatCfg<N>::L * P::T;
+    static constexpr size_t splat = (size_t)SplatCfg<N>::L * SplatCfg<N>::SROW * 8 + NTS * 16 +
                                     kKnotWords * 4 + ((NTS + 31) / 32 + 1) * 4;
     template <int V, int EV = 0>
     static constexpr size_t col() { return (size_t)ColCfg<N, V, EV>::C * FftPlan<N, EV>::PADN * 8 + 16; }
@@ -145,7 +145,7 @@ struct Launch {
     {
         static std::once_flag f;
         set_smem(k_row_splat<N, kSplatTrans>, Smem<N>::splat, f);
-        const int L = RowCfg<N>::L;
+        const int L = SplatCfg<N>::L;
         k_row_splat<N, kSplatTrans><<<nunits * row_blocks(g, L), L * P::T, Smem<N>::splat, s>>>(
             g, units, slice, nsl1, slice_off, atoms, tbuf, nullptr, 0);
     }
@@ -155,7 +155,7 @@ struct Launch {
     {
         static std::once_flag f;
         set_smem(k_row_splat<N, kSplatPot>, Smem<N>::splat, f);
-        const int L = RowCfg<N>::L;
+        const int L = SplatCfg<N>::L;
         k_row_splat<N, kSplatPot><<<nunits * row_blocks(g, L), L * P::T, Smem<N>::splat, s>>>(
             g, units, slice, nsl1, slice_off, atoms, nullptr, vout, vstride);
     }
@@ -165,7 +165,7 @@ struct Launch {
     {
         static std::once_flag f;
         set_smem(k_row_splat<N, kSplatSpec>, Smem<N>::splat, f);
-        const int L = RowCfg<N>::L;
+        const int L = SplatCfg<N>::L;
         k_row_splat<N, kSplatSpec><<<nunits * row_blocks(g, L), L * P::T, Smem<N>::splat, s>>>(
             g, units, slice, nsl1, slice_off, atoms, spec, nullptr, 0);
     }

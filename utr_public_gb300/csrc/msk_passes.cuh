@@ -137,7 +137,7 @@ __device__ __forceinline__ float scat_dI(float2 phi)
 // Rows (lines of length NY) per CTA for the row passes.
 template <int NY> struct RowCfg {
     static constexpr int T = FftPlan<NY>::T;
-    static constexpr int L = (256 / T) > 0 ? 256 / T : 1;   // P1 and most row utilities
+    static constexpr int L = (256 / T) > 0 ? 256 / T : 1;   // most row utilities
     static constexpr int LT = (128 / T) > 0 ? 128 / T : 1;  // the adjoint transmit, k_row_expv
     static constexpr bool BLK = T > 32;
     // resident CTAs per SM the latency-bound utilities are compiled for
@@ -256,15 +256,26 @@ __device__ __forceinline__ float spline_vz(const float *knots, const float4 *coe
 //   Longer lines (a row spans several warps): the atoms touching the CTA's
 //   rows are staged into shared memory in slice order (ordered block
 //   compaction) and every row's threads loop over them.
+// Bound: issue and the latency of the atom loop (60% of issue slots).  Of the
+// 22.3 ms that 48 orientations of 1024^2 take (24.3 ms when every pixel was read
+// back and tested and empty rows went through the phase and shared memory): 9.1
+// rows without any atom (5.8 at the HBM rate), 5.1 the spline at the atoms'
+// pixels, 3.3 the transform, 3.0 the scan and broadcast of atoms, 1.7 exp(i x).
 // MODE kSplatTrans: A = S(exp(i sigma v)), in-band row segments to tbuf
 //      kSplatPot:   v itself (float) to vout + u * vstride
 //      kSplatSpec:  S(v) (v as a complex field), whole rows to tbuf (the
 //                   Debye-Waller branch filters it before the phase)
 enum { kSplatTrans = 0, kSplatPot = 1, kSplatSpec = 2 };
 
-// Per-row shared-memory stride of the splat (float2 units): the padded line,
-// rounded to an even count so every row starts 16-byte aligned (bulk copies).
+// The splat's CTAs: 128 threads, 24 warps an SM (the 80 registers allow no more).
+// Wider ones wait for their slowest row: 256 threads took 5.6 ms against 4.8 (80
+// orientations of 512^2) and 21.0 against 17.8 (a dense 2048^2 specimen).
+// SROW: a row's shared-memory stride (float2 units): the padded line, rounded to
+// an even count so every row starts 16-byte aligned (bulk copies).
 template <int NY> struct SplatCfg {
+    static constexpr int T = FftPlan<NY>::T;
+    static constexpr int L = (128 / T) > 0 ? 128 / T : 1;  // rows per CTA
+    static constexpr int MB = L * T == 128 ? 6 : 1;
     static constexpr int SROW = (FftPlan<NY>::PADN + 1) & ~1;
 };
 
@@ -292,13 +303,39 @@ __device__ __forceinline__ void splat_atom(const Geom &g, const SplatAtom &sa, i
     }
 }
 
+// The groups of T pixels (bit m: iy / T = m) the window of atom `sa` reaches.
+template <int NY, int EV>
+__device__ __forceinline__ unsigned splat_groups(const Geom &g, const SplatAtom &sa)
+{
+    constexpr int T = FftPlan<NY, EV>::T, E = FftPlan<NY, EV>::E, LT = ilog2(T);
+    constexpr unsigned ALL = E == 32 ? 0xffffffffu : (1u << E) - 1u;
+    const int iyo = (int)((sa.meta >> kMetaBits) & kMetaMask);
+    const int g0 = (iyo - g.idy) >> LT, n = ((iyo + g.idy) >> LT) - g0 + 1;
+    if (n >= E) return ALL;
+    const unsigned run = (1u << n) - 1u;
+    const int at = g0 & (E - 1);
+    return ((run << at) | (at ? run >> (E - at) : 0u)) & ALL;
+}
+
+// Zeros over a row's NY potentials, by its T threads.
+template <int NY, int EV>
+__device__ __forceinline__ void splat_zero(float *vacc, int t)
+{
+    constexpr int T = FftPlan<NY, EV>::T, E = FftPlan<NY, EV>::E;
+#pragma unroll
+    for (int m = 0; m < E / 4; m++)
+        reinterpret_cast<float4 *>(vacc)[t + m * T] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+}
+
 // The atoms [a0, a1) of a (unit, slice) whose window touches this warp's RW
 // rows (from wx0), added to the pixels of the row each thread owns (lines of
 // <= 32 threads): the list is scanned 32 atoms at a time, a ballot picks the
 // atoms that touch the warp's rows, each is broadcast by shuffles; per pixel
 // the sums keep the atom order.  vacc = this thread's row (float), zeroed.
+// Returns the groups of T pixels (bit m: iy / T = m) that the windows of those
+// atoms reach; every other group of the warp's rows still holds zeros.
 template <int NY, int EV = 0>
-__device__ __forceinline__ void splat_scan_warp(const Geom &g, const SplatAtom *__restrict__ atoms,
+__device__ __forceinline__ unsigned splat_scan_warp(const Geom &g, const SplatAtom *__restrict__ atoms,
                                                 int a0, int a1, int wx0, int RW, int ix,
                                                 bool row_ok, int t, float *vacc,
                                                 const float *s_knots)
@@ -306,12 +343,15 @@ __device__ __forceinline__ void splat_scan_warp(const Geom &g, const SplatAtom *
     constexpr int T = FftPlan<NY, EV>::T;
     const int nx = g.nx, lane = threadIdx.x & 31;
     const int W = 2 * g.idx + 1;
+    unsigned groups = 0;
+    // the next 32 atoms are requested before the hits of the current ones run
+    SplatAtom ahead = {};
+    if (a0 + lane < a1) ahead = atoms[a0 + lane];
     for (int base = a0; base < a1; base += 32) {
-        const int a = base + lane;
+        const SplatAtom at = ahead;
+        if (base + 32 + lane < a1) ahead = atoms[base + 32 + lane];
         bool hit = false;
-        SplatAtom at = {};
-        if (a < a1) {
-            at = atoms[a];
+        if (base + lane < a1) {
             const int ixo = (int)(at.meta & kMetaMask);
             const int rel = pmod(ixo - g.idx - wx0, nx);
             hit = (W >= nx) || (rel < RW) || (rel + W > nx);
@@ -325,30 +365,30 @@ __device__ __forceinline__ void splat_scan_warp(const Geom &g, const SplatAtom *
             sa.fy = __shfl_sync(0xffffffffu, at.fy, k);
             sa.occ = __shfl_sync(0xffffffffu, at.occ, k);
             sa.meta = __shfl_sync(0xffffffffu, at.meta, k);
+            groups |= splat_groups<NY, EV>(g, sa);
             if (row_ok) splat_atom(g, sa, ix, t, T, NY, W, vacc, s_knots);
         }
     }
     __syncwarp();
+    return groups;
 }
 
 // A = S(exp(i sigma v)) of this thread's row from its potential vacc (float;
 // the row's shared region, which the transform then uses as its exchange
-// buffer): exp(i 0) = 1 exactly where the potential is 0, and rows without
-// atoms take S(1) = NY at iy = 0 directly (what the transform of ones gives).
+// buffer).  Only the pixel groups that atoms reached (splat_scan_warp) are read;
+// elsewhere v = 0 and exp(i 0) = 1.  Rows without atoms take S(1) = NY at iy = 0
+// directly (what the transform of ones gives).
 template <int NY, int SYNC, int EV = 0>
-__device__ __forceinline__ void trans_row(const Geom &g, int t, const float *vacc, float2 *xbuf,
-                                          float2 (&v)[FftPlan<NY, EV>::E])
+__device__ __forceinline__ void trans_row(const Geom &g, int t, unsigned groups, const float *vacc,
+                                          float2 *xbuf, float2 (&v)[FftPlan<NY, EV>::E])
 {
     constexpr int T = FftPlan<NY, EV>::T, E = FftPlan<NY, EV>::E;
-    bool nz = false;
 #pragma unroll
     for (int m = 0; m < E; m++) {
-        const float ph = vacc[t + m * T] * g.sigma_f;
         v[m] = make_float2(1.0f, 0.0f);
-        nz |= ph != 0.0f;
-        if (__any_sync(0xffffffffu, ph != 0.0f)) v[m] = expi(ph);
+        if (groups >> m & 1) v[m] = expi(vacc[t + m * T] * g.sigma_f);
     }
-    if (group_none<SYNC == 1>(nz)) {
+    if (group_none<SYNC == 1>(groups != 0)) {
 #pragma unroll
         for (int m = 0; m < E; m++) v[m] = make_float2(m == 0 && t == 0 ? (float)NY : 0.0f, 0.0f);
     } else {
@@ -401,13 +441,13 @@ __device__ __forceinline__ void warp_store_rows(float2 *rows_smem, int stride, i
 }
 
 template <int NY, int MODE>
-__global__ void __launch_bounds__(RowCfg<NY>::L * FftPlan<NY>::T)
+__global__ void __launch_bounds__(SplatCfg<NY>::L * FftPlan<NY>::T, SplatCfg<NY>::MB)
 k_row_splat(const Geom g, const int *__restrict__ units, int slice, int nsl1,
             const int *__restrict__ slice_off, const SplatAtom *__restrict__ atoms,
             float2 *__restrict__ tbuf, float *__restrict__ vout, size_t vstride)
 {
     using P = FftPlan<NY>;
-    constexpr int T = P::T, E = P::E, L = RowCfg<NY>::L, NT = L * T, NW = (NT + 31) / 32;
+    constexpr int T = P::T, E = P::E, L = SplatCfg<NY>::L, NT = L * T, NW = (NT + 31) / 32;
     constexpr int SROW = SplatCfg<NY>::SROW;
     constexpr bool BLK = RowCfg<NY>::BLK;
     constexpr int RW = BLK ? 1 : 32 / T;  // rows per warp (lines of <= 32 threads)
@@ -428,21 +468,22 @@ k_row_splat(const Geom g, const int *__restrict__ units, int slice, int nsl1,
 
     for (int i = tid; i < kKnotWords; i += NT) s_knots[i] = g.knots[i];
     float *vacc = reinterpret_cast<float *>(s_lines + l * SROW);
-#pragma unroll
-    for (int m = 0; m < E; m++) vacc[t + m * T] = 0.0f;
+    splat_zero<NY, 0>(vacc, t);
     __syncthreads();
 
     const int a0 = slice_off[u * nsl1 + slice], a1 = slice_off[u * nsl1 + slice + 1];
     const int W = 2 * g.idx + 1;
+    unsigned groups = 0;
     if constexpr (!BLK) {
-        splat_scan_warp<NY>(g, atoms, a0, a1, ix0 + warp * RW, RW, ix, row_ok, t, vacc, s_knots);
+        groups = splat_scan_warp<NY>(g, atoms, a0, a1, ix0 + warp * RW, RW, ix, row_ok, t, vacc, s_knots);
     } else {
+        SplatAtom ahead = {};
+        if (a0 + tid < a1) ahead = atoms[a0 + tid];
         for (int base = a0; base < a1; base += NT) {
-            const int a = base + tid;
+            const SplatAtom at = ahead;
+            if (base + NT + tid < a1) ahead = atoms[base + NT + tid];
             bool hit = false;
-            SplatAtom at;
-            if (a < a1) {
-                at = atoms[a];
+            if (base + tid < a1) {
                 const int ixo = (int)(at.meta & kMetaMask);
                 const int rel = pmod(ixo - g.idx - ix0, nx);
                 hit = (W >= nx) || (rel < L) || (rel + W > nx);
@@ -466,7 +507,10 @@ k_row_splat(const Geom g, const int *__restrict__ units, int slice, int nsl1,
             const int nsel = s_cnt[NW];
             __syncthreads();
             if (row_ok)
-                for (int k = 0; k < nsel; k++) splat_atom(g, s_atoms[k], ix, t, T, NY, W, vacc, s_knots);
+                for (int k = 0; k < nsel; k++) {
+                    groups |= splat_groups<NY, 0>(g, s_atoms[k]);
+                    splat_atom(g, s_atoms[k], ix, t, T, NY, W, vacc, s_knots);
+                }
             __syncthreads();
         }
     }
@@ -509,22 +553,29 @@ k_row_splat(const Geom g, const int *__restrict__ units, int slice, int nsl1,
                                 tbuf + ((size_t)u * nx + ix0 + wrow0) * NY);
         }
     } else {
+        float2 *dst = tbuf + ((size_t)u * nx + ix0 + wrow0) * NY;
+        if (!BLK && groups == 0) {  // no atom: S(1), straight from registers
+            for (int r = 0; r < wrows; r++) {
+                float4 *row = reinterpret_cast<float4 *>(dst + (size_t)r * NY);
+                for (int i = lane; i < NY / 2; i += 32)
+                    if (2 * i < g.seg_e1 || 2 * i >= g.seg_s2)
+                        row[i] = make_float4(i == 0 ? (float)NY : 0.0f, 0.0f, 0.0f, 0.0f);
+            }
+            return;
+        }
         float2 v[E];
-        trans_row<NY, BLK ? 1 : 0>(g, t, vacc, s_lines + l * SROW, v);
+        trans_row<NY, BLK ? 1 : 0>(g, t, groups, vacc, s_lines + l * SROW, v);
         // dense rows into shared memory, then their in-band segments to the
         // buffer (its out-of-band columns hold zeros: the band limit zeroes them)
-        if constexpr (BLK) {
-            __syncthreads();
+        const bool tight = g.seg_e1 <= 11 * NY / 32 && g.seg_s2 >= 21 * NY / 32;
+        float2 *row = s_lines + l * (BLK ? NY : SROW);
+        if constexpr (BLK) __syncthreads();
+        else __syncwarp();  // the row's reads of its region are done
 #pragma unroll
-            for (int m = 0; m < E; m++) s_lines[l * NY + t + m * T] = v[m];
-            store_band_rows<NY>(g, s_lines, wrows, tbuf + ((size_t)u * nx + ix0) * NY);
-        } else {
-            __syncwarp();  // the row's reads of its region are done
-#pragma unroll
-            for (int m = 0; m < E; m++) s_lines[l * SROW + t + m * T] = v[m];
-            warp_store_band_rows<NY>(g, s_lines + wrow0 * SROW, SROW, wrows,
-                                     tbuf + ((size_t)u * nx + ix0 + wrow0) * NY);
-        }
+        for (int m = 0; m < E; m++)
+            if (!(E == 32 && band_zero<E>(m) && tight)) row[t + m * T] = v[m];
+        if constexpr (BLK) store_band_rows<NY>(g, s_lines, wrows, dst);
+        else warp_store_band_rows<NY>(g, s_lines + wrow0 * SROW, SROW, wrows, dst);
     }
 }
 

@@ -143,14 +143,13 @@ k_small_slices(const Geom g, int nslices, int nsl1, const int *__restrict__ slic
         } else if (has_n) {  // A_{k+1} = S(exp(i sigma v)) on this row
             float2 *xb = sm + C::ROW0 + rl * C::SROW;
             float *vacc = reinterpret_cast<float *>(xb);
-#pragma unroll
-            for (int m = 0; m < E; m++) vacc[rt + m * T] = 0.0f;
+            splat_zero<N, EV>(vacc, rt);
             __syncwarp();
             const int wx0 = rank * LPC + ((ht >> 5) * C::RW);  // this warp's first row
-            splat_scan_warp<N, EV>(g, atoms, so[k + 1], so[k + 2], wx0, C::RW, row, true, rt,
-                                   vacc, s_knots);
+            const unsigned groups = splat_scan_warp<N, EV>(g, atoms, so[k + 1], so[k + 2], wx0, C::RW,
+                                                           row, true, rt, vacc, s_knots);
             float2 v[E];
-            trans_row<N, 0, EV>(g, rt, vacc, xb, v);
+            trans_row<N, 0, EV>(g, rt, groups, vacc, xb, v);
             float2 *arow = Tu[tb_next] + (size_t)row * N;
 #pragma unroll
             for (int m = 0; m < E; m++)
