@@ -93,6 +93,7 @@ struct msk_context {
     cudaStream_t own_stream = nullptr;  // created with the context
     cudaStream_t aux = nullptr;         // second stream: the wave chain of the slice loop,
                                         // the potential stacks' copies in
+    cudaStream_t aux_first = nullptr;   // the same for small waves: of the highest priority
     cudaStream_t aux2 = nullptr;        // third stream: the potential stacks' copies out
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_t[2] = {}, ev_free[2] = {};
     bool prof_on = false;
@@ -109,6 +110,7 @@ struct msk_context {
     msk::DevBuf stk, stk_v, stk_g, stk_t, stk_img, stk_part, adjtab;  // potential stacks, adjoint
     msk::DevBuf arena;                                // specimen batches
     msk::DevBuf dwbuf;                                // Debye-Waller -B/4 per (unit, slice)
+    msk::DevBuf spec;                                 // Debye-Waller: potentials' spectra
     msk::DevBuf imgfill;                              // image-plane fill values per unit
     msk::DevBuf tune;                                 // scratch grids of the schedule tuners
     msk::DevBuf utr_img, utr_k2, utr_acc, utr_vol, utr_out, utr_tab, utr_stage;  // UTR reconstruction
@@ -123,7 +125,8 @@ struct msk_context {
     std::vector<cudaEvent_t> stk_sev;                 // the same per slice (2 per slice)
     std::vector<cudaStream_t> lanes;                  // concurrent specimens of a batch
     std::vector<cudaEvent_t> lane_ev;                 // lane joins (one per lane) + fork
-    size_t units_alloc = 0;  // units the psi / tbuf buffers hold
+    size_t units_alloc = 0;  // units the psi buffer holds, and at least as many grids
+    size_t group_grids = 0;  // the transmission buffers (0: just units_alloc)
     // msk_calculate's grid and tables as last uploaded (its grid parameters
     // and atomic numbers): repeated calls on one grid skip their preparation;
     // any other upload of the tables clears it

@@ -630,6 +630,7 @@ static bool grid_pre(GridPre &gp, int nx, int ny, float ax, float by, float v0, 
         g.cb_hi0[v] = std::max(g.cb_lo[v], gp.band_q / C);
         g.cb_n[v] = g.cb_lo[v] + (nblk - g.cb_hi0[v]);
     }
+    g.group_units = 1 << 30;  // no groups
     g.seg_e1 = std::min(ny, (gp.band_p + 2) & ~1);
     g.seg_s2 = std::max(g.seg_e1, gp.band_q & ~1);
     return true;
@@ -1397,6 +1398,10 @@ struct Batch {
     std::vector<int> slice_off;   // [nunits][nslices+1] absolute atom offsets
     std::vector<int> act_off;     // [nslices+1]
     std::vector<int> act;         // active units per slice
+    // Slices in groups whose transmissions are made in one launch per pass:
+    // group j holds slices [gstart[j], gstart[j+1]); actv: act's entries as grids
+    // of the group's buffer, (slice - group's first) * nunits + unit
+    std::vector<int> gstart, actv;
     std::vector<float> dw;        // Debye-Waller branch: [nunits][nslices] -B/4 (else empty)
 };
 
@@ -1427,6 +1432,8 @@ size_t pack_batch_meta(const std::vector<UnitAtoms> &ua, int u0, int nunits, int
             if (ua[u0 + i].counts[s] > 0) b.act.push_back(i);
     }
     b.act_off[nslices] = (int)b.act.size();
+    b.gstart.clear();
+    b.actv.clear();
     b.dw.clear();
     if (nunits > 0 && !ua[u0].dw.empty()) {
         b.dw.assign((size_t)nunits * nslices, 0.0f);
@@ -1447,6 +1454,21 @@ void pack_atoms(const std::vector<UnitAtoms> &ua, int u0, const Batch &b, SplatA
         const auto &a = ua[u0 + i].atoms;
         std::copy(a.begin(), a.end(), dst + b.slice_off[(size_t)i * nsl1]);
     });
+}
+
+// The slices of the batch in groups of up to G, the first of a quarter (the wave
+// chain waits for it alone).
+void group_slices(Batch &b, int G)
+{
+    b.gstart.assign(1, 0);
+    b.actv = b.act;
+    if (b.nslices == 0) return;
+    b.gstart.push_back(std::min(b.nslices, std::max(1, G / 4)));
+    while (b.gstart.back() < b.nslices) b.gstart.push_back(std::min(b.nslices, b.gstart.back() + G));
+    for (size_t j = 0; j + 1 < b.gstart.size(); j++)
+        for (int sl = b.gstart[j]; sl < b.gstart[j + 1]; sl++)
+            for (int i = b.act_off[sl]; i < b.act_off[sl + 1]; i++)
+                b.actv[i] += (sl - b.gstart[j]) * b.nunits;
 }
 
 void pack_batch(const std::vector<UnitAtoms> &ua, int u0, int nunits, int nslices, Batch &b,
@@ -1477,12 +1499,17 @@ void *host_stage(msk_context *ctx, size_t bytes)
     return ctx->h_stage;
 }
 
+// group > 1: slices in groups of up to that many (their lists follow the active
+// units on the device).
 int upload_batch(msk_context *ctx, const std::vector<UnitAtoms> &ua, int u0, int nunits,
-                 int nslices, Batch &b)
+                 int nslices, Batch &b, int group = 1)
 {
     const size_t na = std::max<size_t>(pack_batch_meta(ua, u0, nunits, nslices, b), 1);
+    if (group > 1) group_slices(b, group);
+    std::vector<int> lists = b.act;
+    lists.insert(lists.end(), b.actv.begin(), b.actv.end());
     const size_t ab = na * sizeof(SplatAtom), ob = b.slice_off.size() * sizeof(int),
-                 cb = b.act.size() * sizeof(int);
+                 cb = lists.size() * sizeof(int);
     MSK_CUDA(ctx, ctx->atoms.reserve(ab));
     MSK_CUDA(ctx, ctx->slice_off.reserve(ob));
     MSK_CUDA(ctx, ctx->act.reserve(std::max<size_t>(cb, sizeof(int))));
@@ -1491,12 +1518,12 @@ int upload_batch(msk_context *ctx, const std::vector<UnitAtoms> &ua, int u0, int
     // driver's pageable bounce buffers with the GPU idle), else from vectors
     std::vector<SplatAtom> atoms;
     const SplatAtom *src_atoms;
-    const int *src_off = b.slice_off.data(), *src_act = b.act.data();
+    const int *src_off = b.slice_off.data(), *src_act = lists.data();
     if (unsigned char *st = static_cast<unsigned char *>(host_stage(ctx, ab + ob + cb))) {
         SplatAtom *dst = reinterpret_cast<SplatAtom *>(st);
         pack_atoms(ua, u0, b, dst, host_threads());
         std::memcpy(st + ab, b.slice_off.data(), ob);
-        if (cb) std::memcpy(st + ab + ob, b.act.data(), cb);
+        if (cb) std::memcpy(st + ab + ob, lists.data(), cb);
         src_atoms = dst;
         src_off = reinterpret_cast<const int *>(st + ab);
         src_act = reinterpret_cast<const int *>(st + ab + ob);
@@ -1520,6 +1547,23 @@ int upload_batch(msk_context *ctx, const std::vector<UnitAtoms> &ua, int u0, int
     return MSK_OK;
 }
 
+// Slices per group for a batch of `nunits` units of `plane` points, whose
+// transmission buffers hold `grids` grids: about kGroupPoints points a launch.
+// Measured without groups, with launches of 2^23, 2^24, 2^25 and 2^26 points:
+// 45 Debye-Waller units of 256^2 7.8, 6.9, 7.3, 7.0, 7.3 ms; 80 units of 512^2
+// 16.1, 16.3, 15.8, 16.0, 16.3; one of 512^2 2.68, 2.15, 2.19, 2.19, 2.27 (its 64
+// splats together 1.32 ms, then 0.09); 16 of 1024^2 fill launches of their own.
+// nmode 1 and 2 read whole rows of the transmissions, whose out-of-band columns
+// are zeroed for one grid per unit only: no groups.
+constexpr size_t kGroupPoints = (size_t)1 << 24;
+constexpr size_t kFirstPoints = (size_t)1 << 23;  // run_slices: the wave chain goes first
+static int group_size(size_t plane, int nunits, int nslices, int nmode, size_t grids)
+{
+    if (nmode != 0 || nunits < 1 || nslices < 2) return 1;
+    const size_t want = std::min(kGroupPoints / plane, grids) / (size_t)nunits;
+    return (int)std::max<size_t>(1, std::min<size_t>(want, nslices));
+}
+
 // The slice loop over a batch: the psi buffer holds W0 = S(wave0) on entry
 // and W = S(exit wave) on return.
 //
@@ -1529,8 +1573,34 @@ int upload_batch(msk_context *ctx, const std::vector<UnitAtoms> &ua, int u0, int
 // stream while the wave chain of the current one runs on the second stream,
 // so the compute-bound splat overlaps the memory-bound wave passes.  Events
 // order P3 after its P2 and the reuse of a transmission buffer after the P3
-// that read it.  With per-kernel profiling on, everything runs in order on
+// that read it.  The transmissions do not depend on the wave: with few units in
+// the batch those of a group of slices (Batch::gstart) are made in one launch
+// per pass, so that the chain runs at the rate of full launches instead of one
+// launch's latency per slice.  With per-kernel profiling on, everything runs in order on
 // one stream so that each launch is timed alone.
+// The transmission buffers (two sets, and the Debye-Waller branch's spectra) of
+// `grids` grids each; `grids` becomes `units`, one per unit and no groups, where
+// the device has no memory for more.
+static int reserve_transmissions(msk_context *ctx, size_t plane, size_t units, size_t &grids, bool spec)
+{
+    for (;;) {
+        cudaError_t e = ctx->tbuf.reserve(grids * plane * sizeof(float2));
+        if (e == cudaSuccess) e = ctx->tbuf2.reserve(ctx->tbuf.cap);
+        if (e == cudaSuccess && spec) e = ctx->spec.reserve(ctx->tbuf.cap);
+        ctx->group_grids = grids;
+        if (e == cudaSuccess) return MSK_OK;
+        if (e != cudaErrorMemoryAllocation || grids <= units) {
+            MSK_CUDA(ctx, e);
+            return MSK_ECUDA;
+        }
+        cudaGetLastError();  // not sticky: fewer grids
+        ctx->tbuf.release();
+        ctx->tbuf2.release();
+        ctx->spec.release();
+        grids = units;
+    }
+}
+
 // Whether the slice loop of this grid runs as one cluster launch (msk_small.cuh):
 // square grids of 64^2 to 256^2 in the coherent branch with two transmission
 // buffers, on a device that fits the clusters.  MSK_SMALL_GRID=0 in the
@@ -1570,30 +1640,41 @@ int run_slices(msk_context *ctx, const GridPre &gp, const Batch &b, int nmode, b
                                         ctx->tbuf2.as<float2>(), ctx->stream));
         return MSK_OK;
     }
-    // Debye-Waller branch: the second transmission buffer holds the potential's
-    // spectrum, so the two slice chains run in order on one stream
     const bool dw = !b.dw.empty();
-    if (dw && ctx->tbuf2.cap < ctx->tbuf.cap)
-        return fail(ctx, MSK_EUNSUPPORTED, "the Debye-Waller branch needs a second buffer");
-    const bool overlap = !dw && !ctx->prof_on && ctx->tbuf2.cap >= ctx->tbuf.cap;
-    cudaStream_t sA = ctx->stream, sB = overlap ? ctx->aux : ctx->stream;
+    if (dw && ctx->spec.cap < ctx->tbuf.cap)
+        return fail(ctx, MSK_EUNSUPPORTED, "the Debye-Waller branch needs a buffer of its own");
+    const bool overlap = !ctx->prof_on && ctx->tbuf2.cap >= ctx->tbuf.cap;
+    // launches of the wave chain that do not fill the GPU go first, ahead of the
+    // transmissions of later slices, which have slack (45 units of 256^2 6.5 -> 6.1
+    // ms, one of 1024^2 5.99 -> 5.75); large ones do not (16 of 1024^2: 33.8 -> 34.4)
+    const bool first = (size_t)b.nunits * gp.nx * gp.ny <= kFirstPoints;
+    cudaStream_t sA = ctx->stream, sB = !overlap ? ctx->stream : first ? ctx->aux_first : ctx->aux;
     float2 *psi = ctx->psi.as<float2>();
     float2 *tbs[2] = {ctx->tbuf.as<float2>(), overlap ? ctx->tbuf2.as<float2>() : ctx->tbuf.as<float2>()};
     const int *act = ctx->act.as<int>();
     const int nsl1 = b.nslices + 1;
+    // without groups every slice is a group of its own
+    std::vector<int> gstart = b.gstart;
+    const bool grouped = !gstart.empty();
+    if (!grouped)
+        for (int sl = 0; sl <= b.nslices; sl++) gstart.push_back(sl);
+    const int *actv = grouped ? act + b.act.size() : act;
+    Geom gg = g;
+    if (grouped) gg.group_units = b.nunits;
+    const size_t grids = std::max(ctx->units_alloc, ctx->group_grids);
     ColView tmaps[2], pmap;
     const int vm = col_variant(ctx, gp, kColMask), vp = col_variant(ctx, gp, kColProp);
     const int rv = row_variant(ctx, gp);
-    int st = column_map(ctx, &tmaps[0], tbs[0], gp.nx, gp.ny, ctx->units_alloc, cop, vm);
+    int st = column_map(ctx, &tmaps[0], tbs[0], gp.nx, gp.ny, grids, cop, vm);
     if (st) return st;
-    st = column_map(ctx, &tmaps[1], tbs[1], gp.nx, gp.ny, ctx->units_alloc, cop, vm);
+    st = column_map(ctx, &tmaps[1], tbs[1], gp.nx, gp.ny, grids, cop, vm);
     if (st) return st;
     st = column_map(ctx, &pmap, psi, gp.nx, gp.ny, ctx->units_alloc, cop, vp);
     if (st) return st;
     ColView smap;
+    float2 *spec = ctx->spec.as<float2>();
     if (dw) {
-        st = column_map(ctx, &smap, ctx->tbuf2.p, gp.nx, gp.ny, ctx->units_alloc, cop,
-                        col_variant(ctx, gp, kColDW));
+        st = column_map(ctx, &smap, spec, gp.nx, gp.ny, grids, cop, col_variant(ctx, gp, kColDW));
         if (st) return st;
     }
     const double plane = (double)gp.nx * gp.ny;
@@ -1603,58 +1684,64 @@ int run_slices(msk_context *ctx, const GridPre &gp, const Batch &b, int nmode, b
     }
     bool pending_free[2] = {false, false};
     int uses = 0;
-    for (int sl = 0; sl < b.nslices; sl++) {
-        const int na = b.act_off[sl + 1] - b.act_off[sl];
-        const int *units = act + b.act_off[sl];
+    for (size_t j = 0; j + 1 < gstart.size(); j++) {
+        const int s0 = gstart[j], s1 = gstart[j + 1];
+        const int na = b.act_off[s1] - b.act_off[s0];  // grids of the group
+        const int *grid_list = actv + b.act_off[s0];
+        const int k = overlap && na > 0 ? (uses++ & 1) : 0;
+        float2 *tb = tbs[k];
         if (na > 0) {
-            const int k = overlap ? (uses++ & 1) : 0;
-            float2 *tb = tbs[k];
             if (overlap && pending_free[k]) MSK_CUDA(ctx, cudaStreamWaitEvent(sA, ctx->ev_free[k], 0));
             if (dw) {  // trlayerDW: S(v), damping, then A = S(exp(i sigma v'))
-                float2 *spec = ctx->tbuf2.as<float2>();
                 {
                     Prof p(ctx, kSplat, 8.0 * plane * na, sA);
-                    rop->splat_spec(g, units, na, sl, nsl1, ctx->slice_off.as<int>(),
+                    rop->splat_spec(gg, grid_list, na, s0, nsl1, ctx->slice_off.as<int>(),
                                     ctx->atoms.as<SplatAtom>(), spec, sA);
                 }
                 {
                     Prof p(ctx, kDW, 16.0 * plane * na, sA);
-                    cop->col_dw(g, smap, units, na, ctx->dwbuf.as<float>() + sl, b.nslices, sA);
+                    cop->col_dw(gg, smap, grid_list, na, ctx->dwbuf.as<float>() + s0, b.nslices, sA);
                 }
                 Prof p(ctx, kDWExp, 16.0 * plane * na, sA);
-                rop->row_dwexp(g, units, na, spec, tb, sA);
+                rop->row_dwexp(g, grid_list, na, spec, tb, sA);
             } else {
                 Prof p(ctx, kSplat, 8.0 * plane * na, sA);
-                rop->splat(g, units, na, sl, nsl1, ctx->slice_off.as<int>(),
+                rop->splat(gg, grid_list, na, s0, nsl1, ctx->slice_off.as<int>(),
                            ctx->atoms.as<SplatAtom>(), tb, sA);
             }
             {
                 Prof p(ctx, kKColMask, 16.0 * plane * na, sA);
                 // B = S(t_bl) / ny^2: the transmit's 1/ny^2, exact, carried here
-                cop->col_mask(g, tmaps[k], tmaps[k], units, na, 1,
+                cop->col_mask(g, tmaps[k], tmaps[k], grid_list, na, 1,
                               1.0f / ((float)gp.ny * (float)gp.ny), sA);
             }
             if (overlap) {
                 MSK_CUDA(ctx, cudaEventRecord(ctx->ev_t[k], sA));
                 MSK_CUDA(ctx, cudaStreamWaitEvent(sB, ctx->ev_t[k], 0));
             }
-            {
-                Prof p(ctx, kTransmit, 24.0 * plane * na, sB);
-                rop->row_transmit(g, units, na, tb, psi, psi, 1.0f, nmode == 0 && w_in_band, rv,
-                                  sB);
+        }
+        int last = s1 - 1;  // the group's last slice with atoms: the buffer is read then
+        while (last > s0 && b.act_off[last + 1] == b.act_off[last]) last--;
+        for (int sl = s0; sl < s1; sl++) {
+            const int n = b.act_off[sl + 1] - b.act_off[sl];
+            if (n > 0) {
+                Prof p(ctx, kTransmit, 24.0 * plane * n, sB);
+                rop->row_transmit(g, act + b.act_off[sl], n,
+                                  tb + (size_t)(sl - s0) * b.nunits * gp.nx * gp.ny, psi, psi, 1.0f,
+                                  nmode == 0 && w_in_band, rv, sB);
             }
-            if (overlap) {
+            if (overlap && na > 0 && sl == last) {
                 MSK_CUDA(ctx, cudaEventRecord(ctx->ev_free[k], sB));
                 pending_free[k] = true;
             }
-        }
-        if (nmode == 0) {
-            Prof p(ctx, kKColProp, 16.0 * plane * b.nunits, sB);
-            // band mode once every wave is zero out of band: from the start for
-            // a plane wave, else after one full pass (the transmit leaves zeros
-            // there, but units without atoms in a slice keep their wave)
-            cop->col_prop(g, pmap, pmap, nullptr, b.nunits, w_in_band ? 1 : 0, sB);
-            w_in_band = true;
+            if (nmode == 0) {
+                Prof p(ctx, kKColProp, 16.0 * plane * b.nunits, sB);
+                // band mode once every wave is zero out of band: from the start for
+                // a plane wave, else after one full pass (the transmit leaves zeros
+                // there, but units without atoms in a slice keep their wave)
+                cop->col_prop(g, pmap, pmap, nullptr, b.nunits, w_in_band ? 1 : 0, sB);
+                w_in_band = true;
+            }
         }
     }
     if (overlap) {
@@ -1681,6 +1768,9 @@ int msk_create(int device, msk_context **out)
     cudaError_t e = cudaSetDevice(device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->aux, cudaStreamNonBlocking);
+    int least = 0, greatest = 0;
+    if (e == cudaSuccess) e = cudaDeviceGetStreamPriorityRange(&least, &greatest);
+    if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&ctx->aux_first, cudaStreamNonBlocking, greatest);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->aux2, cudaStreamNonBlocking);
     for (cudaEvent_t *ev : {&ctx->ev_fork, &ctx->ev_join, &ctx->ev_t[0], &ctx->ev_t[1],
                             &ctx->ev_free[0], &ctx->ev_free[1]})
@@ -1701,7 +1791,7 @@ void msk_destroy(msk_context *ctx)
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     prof_collect(ctx);
     for (cudaEvent_t e : ctx->prof_pool) cudaEventDestroy(e);
-    for (DevBuf *b : {&ctx->psi, &ctx->tbuf, &ctx->tbuf2, &ctx->atoms, &ctx->slice_off, &ctx->act, &ctx->tables,
+    for (DevBuf *b : {&ctx->spec, &ctx->psi, &ctx->tbuf, &ctx->tbuf2, &ctx->atoms, &ctx->slice_off, &ctx->act, &ctx->tables,
                       &ctx->imgmeta, &ctx->wave0, &ctx->images, &ctx->exitw, &ctx->fresnel,
                       &ctx->flags, &ctx->pa_v, &ctx->pa_t, &ctx->pa_psi, &ctx->pa_e, &ctx->stk,
                       &ctx->stk_v, &ctx->stk_g, &ctx->stk_t, &ctx->stk_img, &ctx->stk_part,
@@ -1718,6 +1808,7 @@ void msk_destroy(msk_context *ctx)
     for (cudaStream_t l : ctx->lanes) cudaStreamDestroy(l);
     for (cudaEvent_t e : ctx->lane_ev) cudaEventDestroy(e);
     if (ctx->aux) cudaStreamDestroy(ctx->aux);
+    if (ctx->aux_first) cudaStreamDestroy(ctx->aux_first);
     if (ctx->aux2) cudaStreamDestroy(ctx->aux2);
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
     if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
@@ -1924,12 +2015,13 @@ int msk_calculate(msk_context *ctx, float *pix, const float *wave0, const float 
     int st = grid_tables(ctx, gp, key, hit, zlist);
     if (st) return st;
     Batch b;
-    st = upload_batch(ctx, ua, 0, 1, nslices, b);
-    if (st) return st;
     const size_t plane = (size_t)nx * ny;
+    size_t grids = small_grid_ok(ctx, gp, thermal == kThermDW, nmode, 1)
+                       ? 1 : group_size(plane, 1, nslices, nmode, kGroupPoints / plane);
     MSK_CUDA(ctx, ctx->psi.reserve(plane * sizeof(float2)));
-    MSK_CUDA(ctx, ctx->tbuf.reserve(plane * sizeof(float2)));
-    MSK_CUDA(ctx, ctx->tbuf2.reserve(plane * sizeof(float2)));
+    if ((st = reserve_transmissions(ctx, plane, 1, grids, thermal == kThermDW))) return st;
+    st = upload_batch(ctx, ua, 0, 1, nslices, b, (int)grids);
+    if (st) return st;
     // the splat stores in-band row segments only: the rest must read as zeros
     MSK_CUDA(ctx, cudaMemsetAsync(ctx->tbuf.p, 0, plane * sizeof(float2), ctx->stream));
     MSK_CUDA(ctx, cudaMemsetAsync(ctx->tbuf2.p, 0, plane * sizeof(float2), ctx->stream));
@@ -2043,7 +2135,10 @@ int tilt_series_impl(msk_context *ctx, const msk_series *s, int natom, const int
     std::vector<int> bounds = {0};
     {
         int first = B;
-        if (s->max_batch <= 0 && nunits >= 32) {
+        // (worth it when the preparation, about 0.1 us an atom and unit on one host
+        // thread, takes longer than a small batch's slices, about 30 us each)
+        if (s->max_batch <= 0 && nunits >= 32 &&
+            1e-4 * natom * nunits / host_threads() > 0.03 * nslices) {
             first = std::min(B, std::max(8, (nunits + 15) / 16));
             if (nconfig > 1) first = std::max(nconfig, (first / nconfig) * nconfig);
             first = std::min(first, B);
@@ -2084,9 +2179,14 @@ int tilt_series_impl(msk_context *ctx, const msk_series *s, int natom, const int
         ev_ready = ctx->stk_ev[0];
         ev_copied = ctx->stk_ev[1];
     }
+    // grids per transmission buffer: one per unit, or a group of slices of them
+    const bool dw_branch = s->lwobble && nconfig == 1;
+    const bool small = small_grid_ok(ctx, gp, dw_branch, s->nmode, nunits);
+    size_t grids =
+        small ? (size_t)B
+              : std::max<size_t>(B, std::min<size_t>(kGroupPoints / plane, (size_t)B * nslices));
     MSK_CUDA(ctx, ctx->psi.reserve((size_t)B * plane * sizeof(float2)));
-    MSK_CUDA(ctx, ctx->tbuf.reserve((size_t)B * plane * sizeof(float2)));
-    MSK_CUDA(ctx, ctx->tbuf2.reserve((size_t)B * plane * sizeof(float2)));
+    if ((st = reserve_transmissions(ctx, plane, B, grids, dw_branch))) return st;
     // the splat stores in-band row segments only: the rest must read as zeros
     MSK_CUDA(ctx, cudaMemsetAsync(ctx->tbuf.p, 0, (size_t)B * plane * sizeof(float2), ctx->stream));
     MSK_CUDA(ctx, cudaMemsetAsync(ctx->tbuf2.p, 0, (size_t)B * plane * sizeof(float2), ctx->stream));
@@ -2167,7 +2267,8 @@ int tilt_series_impl(msk_context *ctx, const msk_series *s, int natom, const int
             if (ua[u0 + i].status)
                 return fail(ctx, ua[u0 + i].status, msk_status_string(ua[u0 + i].status));
         Batch b;
-        st = upload_batch(ctx, ua, u0, nb, nslices, b);
+        st = upload_batch(ctx, ua, u0, nb, nslices, b,
+                          small ? 1 : group_size(plane, nb, nslices, s->nmode, grids));
         if (st) return st;
         b.call_units = nunits;
         float2 *psi = ctx->psi.as<float2>(), *tb = ctx->tbuf.as<float2>();

@@ -460,7 +460,8 @@ k_row_splat(const Geom g, const int *__restrict__ units, int slice, int nsl1,
     const int tid = threadIdx.x, l = tid / T, t = tid % T;
     const int nx = g.nx;
     const int bpu = (nx + L - 1) / L;
-    const int u = units[blockIdx.x / bpu];
+    const int vu = units[blockIdx.x / bpu];  // the grid written; its unit and slice
+    const int u = vu % g.group_units, sl = slice + vu / g.group_units;
     const int ix0 = (blockIdx.x % bpu) * L;
     const int ix = ix0 + l;
     const bool row_ok = ix < nx;
@@ -471,7 +472,7 @@ k_row_splat(const Geom g, const int *__restrict__ units, int slice, int nsl1,
     splat_zero<NY, 0>(vacc, t);
     __syncthreads();
 
-    const int a0 = slice_off[u * nsl1 + slice], a1 = slice_off[u * nsl1 + slice + 1];
+    const int a0 = slice_off[u * nsl1 + sl], a1 = slice_off[u * nsl1 + sl + 1];
     const int W = 2 * g.idx + 1;
     unsigned groups = 0;
     if constexpr (!BLK) {
@@ -520,7 +521,7 @@ k_row_splat(const Geom g, const int *__restrict__ units, int slice, int nsl1,
     if constexpr (MODE == kSplatPot) {
         // the projected potential itself: vout -> slice `slice` of unit 0
         if (row_ok) {
-            float *dst = vout + (size_t)u * vstride + (size_t)ix * NY;
+            float *dst = vout + (size_t)vu * vstride + (size_t)ix * NY;
 #pragma unroll
             for (int m = 0; m < E; m++) dst[t + m * T] = vacc[t + m * T];
         }
@@ -541,7 +542,7 @@ k_row_splat(const Geom g, const int *__restrict__ units, int slice, int nsl1,
             fence_proxy_async();
             __syncthreads();
             if (tid == 0) {
-                bulk_store(tbuf + ((size_t)u * nx + ix0) * NY, s_lines, (uint32_t)wrows * NY * 8u);
+                bulk_store(tbuf + ((size_t)vu * nx + ix0) * NY, s_lines, (uint32_t)wrows * NY * 8u);
                 bulk_commit();
                 bulk_wait_read();
             }
@@ -550,10 +551,10 @@ k_row_splat(const Geom g, const int *__restrict__ units, int slice, int nsl1,
 #pragma unroll
             for (int m = 0; m < E; m++) s_lines[l * SROW + t + m * T] = v[m];
             warp_store_rows<NY>(s_lines + wrow0 * SROW, SROW, wrows,
-                                tbuf + ((size_t)u * nx + ix0 + wrow0) * NY);
+                                tbuf + ((size_t)vu * nx + ix0 + wrow0) * NY);
         }
     } else {
-        float2 *dst = tbuf + ((size_t)u * nx + ix0 + wrow0) * NY;
+        float2 *dst = tbuf + ((size_t)vu * nx + ix0 + wrow0) * NY;
         if (!BLK && groups == 0) {  // no atom: S(1), straight from registers
             for (int r = 0; r < wrows; r++) {
                 float4 *row = reinterpret_cast<float4 *>(dst + (size_t)r * NY);
@@ -657,7 +658,7 @@ k_col_pass(const Geom g, const __grid_constant__ CUtensorMap in_map,
                                               : make_float2(0.0f, 0.0f);
         }
     } else if constexpr (MODE == kColDW) {
-        const float mb4 = __ldg(&fr.dw[(size_t)u * fr.dw_stride]);
+        const float mb4 = __ldg(&fr.dw[(size_t)(u % g.group_units) * fr.dw_stride + u / g.group_units]);
         const float ky2 = __ldg(&g.ky2[iy]);
 #pragma unroll
         for (int m = 0; m < E; m++) {

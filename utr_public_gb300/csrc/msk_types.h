@@ -41,6 +41,10 @@ struct Geom {
     const float2 *tw_col16;
     const float *knots;    // [100] spline knots in r^2
     const float4 *coef;    // [nz][100] spline {y, b, c, d} per compact atomic number
+    // Grouped slices: an entry of a unit list is v = s * group_units + u, the unit
+    // u in the s-th slice from the launch's, with grid v of the launch's buffer.
+    // Without groups (group_units beyond any list) v is the unit.
+    int group_units;
     int *err;              // device error flags (kErrWaitTimeout ...), 0 when all is well
 };
 
