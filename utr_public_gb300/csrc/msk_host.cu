@@ -969,6 +969,8 @@ int column_map(msk_context *ctx, ColView *view, void *base, int nx, int ny, size
 // synchronisation (a bounded wait in a kernel that gave up sets a bit).
 // The same buffer holds, after 256 bytes, kZeroBytes of zeros: the source
 // the row passes fill out-of-band row segments from.
+// Byte 128 holds the barrier counter of k_wide_wave.
+constexpr size_t kWideCounter = 128;
 constexpr size_t kZeroBytes = 4096 * sizeof(float2);
 constexpr size_t kFlagBytes = 256 + kZeroBytes;
 
@@ -1601,45 +1603,45 @@ static int reserve_transmissions(msk_context *ctx, size_t plane, size_t units, s
     }
 }
 
-// Whether the slice loop of this grid runs as one cluster launch (msk_small.cuh):
-// square grids of 64^2 to 256^2 in the coherent branch with two transmission
-// buffers, on a device that fits the clusters.  MSK_SMALL_GRID=0 in the
-// environment keeps the launch-per-pass loop (=1: the default).
-// Only when the units fit in one wave of clusters: with more, the launch-per-pass
-// loop keeps the whole GPU busy and is faster (64 orientations of a 256^2 specimen:
-// 116k slice-steps/s in clusters against 188k in the loop), while a few units leave
-// the loop's launches latency-bound (C1, one unit: 0.52 ms against ~1 ms).
-static bool small_grid_ok(msk_context *ctx, const GridPre &gp, bool dw, int nmode, int nunits)
+// Whether the wave chain of this grid's slice loop runs as cluster launches
+// (k_small_wave, msk_small.cuh), one per slice group: square grids of 64^2 to
+// 256^2, on a device that fits the clusters.  MSK_SMALL_GRID=0 in the environment
+// keeps the launch-per-pass loop (=1: the default).
+// Only when the units' clusters have an SM a CTA each: with more, the loop keeps
+// the whole GPU busy and is faster (64 orientations of a 256^2 specimen in
+// clusters 116k slice-steps/s against 188k in the loop), while a few units leave
+// the loop's launches latency-bound (one unit of 256^2, 32 slices: 0.18 ms
+// against ~0.5).
+static bool small_grid_ok(msk_context *ctx, const GridPre &gp, int nmode, int nunits)
 {
     const char *forced = getenv("MSK_SMALL_GRID");
     if (forced && forced[0] == '0') return false;
     const SizeOps *op = size_ops(gp.nx);
-    return nmode == 0 && !dw && gp.nx == gp.ny && op && op->small_slices &&
-           nunits <= op->small_ok(ctx->device);
+    return nmode == 0 && gp.nx == gp.ny && op && op->small_wave && nunits <= op->small_ok(ctx->device);
 }
 
 static bool small_path(msk_context *ctx, const GridPre &gp, const Batch &b, int nmode)
 {
     return ctx->tbuf2.cap >= ctx->tbuf.cap && ctx->tbuf.cap > 0 &&
-           small_grid_ok(ctx, gp, !b.dw.empty(), nmode, std::max(b.nunits, b.call_units));
+           small_grid_ok(ctx, gp, nmode, std::max(b.nunits, b.call_units));
+}
+
+// The same for a lone unit of 512^2 or 1024^2 (k_wide_wave): it computes what the
+// launch loop's 32-point plans compute.  MSK_SMALL_GRID=0 keeps the loop here too.
+static bool wide_path(msk_context *ctx, const GridPre &gp, const Batch &b, int nmode)
+{
+    const char *forced = getenv("MSK_SMALL_GRID");
+    if (forced && forced[0] == '0') return false;
+    const SizeOps *op = size_ops(gp.nx);
+    return nmode == 0 && gp.nx == gp.ny && op && op->wide_wave && b.nunits == 1 && b.call_units <= 1 &&
+           ctx->tbuf2.cap >= ctx->tbuf.cap && ctx->tbuf.cap > 0 && op->wide_ok(ctx->device);
 }
 
 int run_slices(msk_context *ctx, const GridPre &gp, const Batch &b, int nmode, bool w_in_band)
 {
     const SizeOps *rop = size_ops(gp.ny), *cop = size_ops(gp.nx);
     const Geom &g = gp.g;
-    if (small_path(ctx, gp, b, nmode)) {
-        // every slice of every unit in one launch; algorithmic bytes as the
-        // passes count them (64 N per slice-step with atoms, 16 N without)
-        const double plane = (double)gp.nx * gp.ny;
-        const double ne = b.act_off[b.nslices], all = (double)b.nunits * b.nslices;
-        Prof p(ctx, kSmall, plane * (64.0 * ne + 16.0 * (all - ne)));
-        MSK_CUDA(ctx, cop->small_slices(g, b.nunits, b.nslices, b.nslices + 1,
-                                        ctx->slice_off.as<int>(), ctx->atoms.as<SplatAtom>(),
-                                        ctx->psi.as<float2>(), ctx->tbuf.as<float2>(),
-                                        ctx->tbuf2.as<float2>(), ctx->stream));
-        return MSK_OK;
-    }
+    const bool small = small_path(ctx, gp, b, nmode), wide = wide_path(ctx, gp, b, nmode);
     const bool dw = !b.dw.empty();
     if (dw && ctx->spec.cap < ctx->tbuf.cap)
         return fail(ctx, MSK_EUNSUPPORTED, "the Debye-Waller branch needs a buffer of its own");
@@ -1663,8 +1665,9 @@ int run_slices(msk_context *ctx, const GridPre &gp, const Batch &b, int nmode, b
     if (grouped) gg.group_units = b.nunits;
     const size_t grids = std::max(ctx->units_alloc, ctx->group_grids);
     ColView tmaps[2], pmap;
-    const int vm = col_variant(ctx, gp, kColMask), vp = col_variant(ctx, gp, kColProp);
-    const int rv = row_variant(ctx, gp);
+    // (the wave chain of a small grid or a lone unit runs without these plans)
+    const int vm = col_variant(ctx, gp, kColMask), vp = small || wide ? 0 : col_variant(ctx, gp, kColProp);
+    const int rv = small || wide ? 0 : row_variant(ctx, gp);
     int st = column_map(ctx, &tmaps[0], tbs[0], gp.nx, gp.ny, grids, cop, vm);
     if (st) return st;
     st = column_map(ctx, &tmaps[1], tbs[1], gp.nx, gp.ny, grids, cop, vm);
@@ -1715,10 +1718,29 @@ int run_slices(msk_context *ctx, const GridPre &gp, const Batch &b, int nmode, b
                 cop->col_mask(g, tmaps[k], tmaps[k], grid_list, na, 1,
                               1.0f / ((float)gp.ny * (float)gp.ny), sA);
             }
+            if (small || wide) {
+                Prof p(ctx, kExit, 16.0 * plane * na, sA);
+                rop->row_band_inverse(g, grid_list, na, tb, sA);
+            }
             if (overlap) {
                 MSK_CUDA(ctx, cudaEventRecord(ctx->ev_t[k], sA));
                 MSK_CUDA(ctx, cudaStreamWaitEvent(sB, ctx->ev_t[k], 0));
             }
+        }
+        if (small || wide) {
+            unsigned *count = reinterpret_cast<unsigned *>(ctx->flags.as<unsigned char>() + kWideCounter);
+            if (wide) MSK_CUDA(ctx, cudaMemsetAsync(count, 0, sizeof(unsigned), sB));
+            Prof p(ctx, kSmall, plane * (24.0 * na + 16.0 * b.nunits * (s1 - s0)), sB);
+            const int *so = ctx->slice_off.as<int>();
+            const int arbitrary = w_in_band ? 0 : 1;
+            MSK_CUDA(ctx, small ? cop->small_wave(g, b.nunits, s0, s1, nsl1, so, tb, psi, arbitrary, sB)
+                                : cop->wide_wave(g, s0, s1, so, tb, psi, arbitrary, count, sB));
+            w_in_band = true;
+            if (overlap && na > 0) {
+                MSK_CUDA(ctx, cudaEventRecord(ctx->ev_free[k], sB));
+                pending_free[k] = true;
+            }
+            continue;
         }
         int last = s1 - 1;  // the group's last slice with atoms: the buffer is read then
         while (last > s0 && b.act_off[last + 1] == b.act_off[last]) last--;
@@ -2016,8 +2038,7 @@ int msk_calculate(msk_context *ctx, float *pix, const float *wave0, const float 
     if (st) return st;
     Batch b;
     const size_t plane = (size_t)nx * ny;
-    size_t grids = small_grid_ok(ctx, gp, thermal == kThermDW, nmode, 1)
-                       ? 1 : group_size(plane, 1, nslices, nmode, kGroupPoints / plane);
+    size_t grids = group_size(plane, 1, nslices, nmode, kGroupPoints / plane);
     MSK_CUDA(ctx, ctx->psi.reserve(plane * sizeof(float2)));
     if ((st = reserve_transmissions(ctx, plane, 1, grids, thermal == kThermDW))) return st;
     st = upload_batch(ctx, ua, 0, 1, nslices, b, (int)grids);
@@ -2181,10 +2202,7 @@ int tilt_series_impl(msk_context *ctx, const msk_series *s, int natom, const int
     }
     // grids per transmission buffer: one per unit, or a group of slices of them
     const bool dw_branch = s->lwobble && nconfig == 1;
-    const bool small = small_grid_ok(ctx, gp, dw_branch, s->nmode, nunits);
-    size_t grids =
-        small ? (size_t)B
-              : std::max<size_t>(B, std::min<size_t>(kGroupPoints / plane, (size_t)B * nslices));
+    size_t grids = std::max<size_t>(B, std::min<size_t>(kGroupPoints / plane, (size_t)B * nslices));
     MSK_CUDA(ctx, ctx->psi.reserve((size_t)B * plane * sizeof(float2)));
     if ((st = reserve_transmissions(ctx, plane, B, grids, dw_branch))) return st;
     // the splat stores in-band row segments only: the rest must read as zeros
@@ -2268,7 +2286,7 @@ int tilt_series_impl(msk_context *ctx, const msk_series *s, int natom, const int
                 return fail(ctx, ua[u0 + i].status, msk_status_string(ua[u0 + i].status));
         Batch b;
         st = upload_batch(ctx, ua, u0, nb, nslices, b,
-                          small ? 1 : group_size(plane, nb, nslices, s->nmode, grids));
+                          group_size(plane, nb, nslices, s->nmode, grids));
         if (st) return st;
         b.call_units = nunits;
         float2 *psi = ctx->psi.as<float2>(), *tb = ctx->tbuf.as<float2>();
@@ -3197,8 +3215,8 @@ struct SpecPlan {
     size_t o_tab = 0, o_atoms = 0, o_soff = 0, o_act = 0, o_meta = 0, o_w0 = 0;  // upload region
     size_t o_fres = 0, o_psi = 0, o_tbuf = 0, o_img = 0, o_phi = 0, o_fill = 0;  // work region
     size_t o_dw = 0, o_spec = 0;  // Debye-Waller branch: -B/4 per (unit, slice); S(v) grids
-    bool small = false;      // the slice loop as one cluster launch (msk_small.cuh)
-    size_t o_tbuf2 = 0;      // its second transmission buffer
+    bool small = false;  // the wave chain as one cluster launch per group (msk_small.cuh)
+    int group = 1;       // slices per group (run_slices)
     bool img_dev = false;
     bool img_pinned = false;  // host images in page-locked memory: copied on the lane
     float *ew = nullptr;      // exit waves out (may be null)
@@ -3247,7 +3265,8 @@ int enqueue_specimen(msk_context *ctx, SpecPlan &P, unsigned char *arena, const 
     ColView pmap, tmap, pmapf, tmapf, smap;
     int rc = column_map(ctx, &pmap, psi, nx, ny, na, cop, vp);
     if (rc) return rc;
-    rc = column_map(ctx, &tmap, tb, nx, ny, na, cop, vm);
+    const size_t grids = (size_t)na * P.group;
+    rc = column_map(ctx, &tmap, tb, nx, ny, grids, cop, vm);
     if (rc) return rc;
     rc = column_map(ctx, &pmapf, psi, nx, ny, na, cop, vf);
     if (rc) return rc;
@@ -3257,7 +3276,7 @@ int enqueue_specimen(msk_context *ctx, SpecPlan &P, unsigned char *arena, const 
     const bool dw = !P.b.dw.empty();
     float2 *spec = reinterpret_cast<float2 *>(arena + P.o_spec);
     const float *dwf = reinterpret_cast<const float *>(arena + P.o_dw);
-    if (dw && (rc = column_map(ctx, &smap, spec, nx, ny, na, cop, col_variant(ctx, gp, kColDW))))
+    if (dw && (rc = column_map(ctx, &smap, spec, nx, ny, grids, cop, col_variant(ctx, gp, kColDW))))
         return rc;
     const double pl = (double)plane;
     // incident wave: a plane wave (in band from the start) or the specimen's
@@ -3272,44 +3291,62 @@ int enqueue_specimen(msk_context *ctx, SpecPlan &P, unsigned char *arena, const 
                       st);
     }
     const int nsl1 = P.nslices + 1;
-    if (P.small) {  // every slice of every unit in one cluster launch, as run_slices
-        const double ne = P.b.act_off[P.nslices], all = (double)na * P.nslices;
-        Prof p(ctx, kSmall, pl * (64.0 * ne + 16.0 * (all - ne)), st);
-        MSK_CUDA(ctx, cop->small_slices(g, na, P.nslices, nsl1, soff, atoms, psi, tb,
-                                        reinterpret_cast<float2 *>(arena + P.o_tbuf2), st));
-    }
-    for (int sl = 0; sl < (P.small ? 0 : P.nslices); sl++) {
-        const int nact = P.b.act_off[sl + 1] - P.b.act_off[sl];
-        const int *units = act + P.b.act_off[sl];
+    // groups of slices as in run_slices, on this one stream (the other specimens'
+    // lanes run beside it)
+    std::vector<int> gstart = P.b.gstart;
+    if (gstart.empty())
+        for (int sl = 0; sl <= P.nslices; sl++) gstart.push_back(sl);
+    const int *actv = P.b.gstart.empty() ? act : act + P.b.act.size();
+    Geom gg = g;
+    if (!P.b.gstart.empty()) gg.group_units = na;
+    for (size_t j = 0; j + 1 < gstart.size(); j++) {
+        const int s0 = gstart[j], s1 = gstart[j + 1];
+        const int nact = P.b.act_off[s1] - P.b.act_off[s0];
+        const int *grid_list = actv + P.b.act_off[s0];
         if (nact > 0) {
             if (dw) {  // S(v), the damping, then A = S(exp(i sigma v')), as run_slices
                 {
                     Prof p(ctx, kSplat, 8.0 * pl * nact, st);
-                    rop->splat_spec(g, units, nact, sl, nsl1, soff, atoms, spec, st);
+                    rop->splat_spec(gg, grid_list, nact, s0, nsl1, soff, atoms, spec, st);
                 }
                 {
                     Prof p(ctx, kDW, 16.0 * pl * nact, st);
-                    cop->col_dw(g, smap, units, nact, dwf + sl, P.nslices, st);
+                    cop->col_dw(gg, smap, grid_list, nact, dwf + s0, P.nslices, st);
                 }
                 Prof p(ctx, kDWExp, 16.0 * pl * nact, st);
-                rop->row_dwexp(g, units, nact, spec, tb, st);
+                rop->row_dwexp(g, grid_list, nact, spec, tb, st);
             } else {
                 Prof p(ctx, kSplat, 8.0 * pl * nact, st);
-                rop->splat(g, units, nact, sl, nsl1, soff, atoms, tb, st);
+                rop->splat(gg, grid_list, nact, s0, nsl1, soff, atoms, tb, st);
             }
             {
                 Prof p(ctx, kKColMask, 16.0 * pl * nact, st);
                 // B = S(t_bl) / ny^2: the transmit's 1/ny^2, exact, carried here
-                cop->col_mask(g, tmap, tmap, units, nact, 1, 1.0f / ((float)ny * (float)ny), st);
+                cop->col_mask(g, tmap, tmap, grid_list, nact, 1, 1.0f / ((float)ny * (float)ny), st);
             }
-            Prof p(ctx, kTransmit, 24.0 * pl * nact, st);
-            rop->row_transmit(g, units, nact, tb, psi, psi, 1.0f, s->nmode == 0 && w_in_band, rv,
-                              st);
+            if (P.small) {
+                Prof p(ctx, kExit, 16.0 * pl * nact, st);
+                rop->row_band_inverse(g, grid_list, nact, tb, st);
+            }
         }
-        if (s->nmode == 0) {
-            Prof p(ctx, kKColProp, 16.0 * pl * na, st);
-            cop->col_prop(g, pmap, pmap, nullptr, na, w_in_band ? 1 : 0, st);
+        if (P.small) {
+            Prof p(ctx, kSmall, pl * (24.0 * nact + 16.0 * na * (s1 - s0)), st);
+            MSK_CUDA(ctx, cop->small_wave(g, na, s0, s1, nsl1, soff, tb, psi, w_in_band ? 0 : 1, st));
             w_in_band = true;
+            continue;
+        }
+        for (int sl = s0; sl < s1; sl++) {
+            const int n = P.b.act_off[sl + 1] - P.b.act_off[sl];
+            if (n > 0) {
+                Prof p(ctx, kTransmit, 24.0 * pl * n, st);
+                rop->row_transmit(g, act + P.b.act_off[sl], n, tb + (size_t)(sl - s0) * na * plane, psi,
+                                  psi, 1.0f, s->nmode == 0 && w_in_band, rv, st);
+            }
+            if (s->nmode == 0) {
+                Prof p(ctx, kKColProp, 16.0 * pl * na, st);
+                cop->col_prop(g, pmap, pmap, nullptr, na, w_in_band ? 1 : 0, st);
+                w_in_band = true;
+            }
         }
     }
     // exit waves (psi = iS(W)/ny): into a device destination directly, else
@@ -3536,7 +3573,11 @@ extern "C" int msk_tilt_series_batch(msk_context *ctx, const msk_series *s, int 
         q.o_soff = up;
         up += align256(q.b.slice_off.size() * sizeof(int));
         q.o_act = up;
-        up += align256(std::max<size_t>(q.b.act.size(), 1) * sizeof(int));
+        q.small = small_grid_ok(ctx, q.gp, s->nmode, q.nunits);
+        q.group = group_size(plane, q.nunits, q.nslices, s->nmode, kGroupPoints / plane);
+        if (q.group > 1 && q.b.gstart.empty()) group_slices(q.b, q.group);
+        const size_t grids = (size_t)q.nunits * q.group;
+        up += align256(std::max<size_t>(q.b.act.size() + q.b.actv.size(), 1) * sizeof(int));
         q.o_meta = up;
         up += align256(std::max<size_t>(q.meta.size(), 1) * sizeof(int));
         q.o_w0 = up;
@@ -3548,10 +3589,7 @@ extern "C" int msk_tilt_series_batch(msk_context *ctx, const msk_series *s, int 
         q.o_psi = work;
         work += align256((size_t)q.nunits * plane * sizeof(float2));
         q.o_tbuf = work;
-        work += align256((size_t)q.nunits * plane * sizeof(float2));
-        q.small = small_grid_ok(ctx, q.gp, !q.b.dw.empty(), s->nmode, q.nunits);
-        q.o_tbuf2 = work;
-        if (q.small) work += align256((size_t)q.nunits * plane * sizeof(float2));
+        work += align256(grids * plane * sizeof(float2));
         q.o_img = work;
         if (!q.img_dev) work += align256((size_t)q.nimages * plane * sizeof(float));
         // a rotated or shifted image plane: a real-space scratch grid per unit and
@@ -3561,7 +3599,7 @@ extern "C" int msk_tilt_series_batch(msk_context *ctx, const msk_series *s, int 
         q.o_fill = work;
         if (q.image_plane) work += align256((size_t)q.nunits * sizeof(float2));
         q.o_spec = work;
-        if (!q.b.dw.empty()) work += align256((size_t)q.nunits * plane * sizeof(float2));
+        if (!q.b.dw.empty()) work += align256(grids * plane * sizeof(float2));
         q.o_ew = work;
         if (q.ew && !q.ew_dev && !q.ew_pinned)
             work += align256((size_t)q.nunits * plane * sizeof(float2));
@@ -3584,7 +3622,6 @@ extern "C" int msk_tilt_series_batch(msk_context *ctx, const msk_series *s, int 
             P[i].o_fres += align256(up);
             P[i].o_psi += align256(up);
             P[i].o_tbuf += align256(up);
-            P[i].o_tbuf2 += align256(up);
             P[i].o_img += align256(up);
             P[i].o_phi += align256(up);
             P[i].o_fill += align256(up);
@@ -3603,6 +3640,9 @@ extern "C" int msk_tilt_series_batch(msk_context *ctx, const msk_series *s, int 
             std::memcpy(&host[q.o_soff], q.b.slice_off.data(), q.b.slice_off.size() * sizeof(int));
             if (!q.b.act.empty())
                 std::memcpy(&host[q.o_act], q.b.act.data(), q.b.act.size() * sizeof(int));
+            if (!q.b.actv.empty())
+                std::memcpy(&host[q.o_act] + q.b.act.size() * sizeof(int), q.b.actv.data(),
+                            q.b.actv.size() * sizeof(int));
             if (!q.meta.empty())
                 std::memcpy(&host[q.o_meta], q.meta.data(), q.meta.size() * sizeof(int));
             if (!q.wave0.empty())

@@ -3,11 +3,13 @@
 // row passes by ny and column passes by nx.
 #pragma once
 
+#include <algorithm>
 #include <mutex>
 
 #include "msk_passes.cuh"
 #include "msk_small.cuh"
 #include "msk_types.h"
+#include "msk_wide.cuh"
 
 namespace msk {
 
@@ -74,6 +76,8 @@ struct SizeOps {
                      float2 *psi, float scale, cudaStream_t);
     void (*row_exit)(const Geom &, const int *units, int nunits, const float2 *psi,
                      float2 *out, cudaStream_t);
+    // buf = iS(buf), its out-of-band columns taken as zeros
+    void (*row_band_inverse)(const Geom &, const int *units, int nunits, float2 *buf, cudaStream_t);
     // out = iS(in) * scale (the real-space wave of a W-state, unnormalised)
     void (*row_inverse)(const Geom &, const int *units, int nunits, const float2 *in,
                         float2 *out, float scale, cudaStream_t);
@@ -93,14 +97,21 @@ struct SizeOps {
     // returns the number of loss partials written
     int (*row_imgrad)(const Geom &, int nunits, const float2 *E, const float *target,
                       size_t tstride, float2 *G, double *partial, cudaStream_t);
-    // square grids of N <= 256: every slice of every unit in one cluster launch
-    // (msk_small.cuh); W holds S(psi) on entry and exit, T0 / T1 scratch of the
-    // same size.  small_ok: how many of its clusters the device runs at once
-    // (0: none fit).  Both null for other sizes.
-    cudaError_t (*small_slices)(const Geom &, int nunits, int nslices, int nsl1,
-                                const int *slice_off, const SplatAtom *atoms, float2 *W,
-                                float2 *T0, float2 *T1, cudaStream_t);
-    int (*small_ok)(int device);  // clusters of this size active at once (0: none fit)
+    // square grids of 64 <= N <= 256 (null for other sizes).  small_ok: how many
+    // units' clusters the device runs at once, an SM a CTA (0: none fit)
+    int (*small_ok)(int device);
+    // the wave chain of slices s0 .. s1-1 alone, from transmissions iS(B) made
+    // beforehand (grid (k - s0) * nunits + u of t); arbitrary: W may hold anything
+    // out of band.
+    cudaError_t (*small_wave)(const Geom &, int nunits, int s0, int s1, int nsl1,
+                              const int *slice_off, const float2 *t, float2 *W, int arbitrary,
+                              cudaStream_t);
+    // the same for one unit of a square 512^2 or 1024^2 grid in one cooperative
+    // launch (msk_wide.cuh); `count` zeroed.  wide_ok: the device holds its CTAs at
+    // once.  Both null for other sizes.
+    cudaError_t (*wide_wave)(const Geom &, int s0, int s1, const int *slice_off, const float2 *t,
+                             float2 *W, int arbitrary, unsigned *count, cudaStream_t);
+    bool (*wide_ok)(int device);
 };
 
 // Line lengths with kernels: 16 .. 4096, powers of two.
@@ -306,6 +317,15 @@ struct Launch {
         k_row_simple<N, kRowInit><<<nunits * row_blocks(g, L), L * P::T, Smem<N>::row, s>>>(
             g, units, wave0, psi, scale);
     }
+    static void row_band_inverse(const Geom &g, const int *units, int nunits, float2 *buf,
+                                 cudaStream_t s)
+    {
+        static std::once_flag f;
+        set_smem(k_row_simple<N, kRowBand>, Smem<N>::row, f);
+        const int L = RowCfg<N>::L;
+        k_row_simple<N, kRowBand><<<nunits * row_blocks(g, L), L * P::T, Smem<N>::row, s>>>(
+            g, units, buf, buf, 1.0f);
+    }
     static void row_inverse(const Geom &g, const int *units, int nunits, const float2 *in,
                             float2 *out, float scale, cudaStream_t s)
     {
@@ -375,7 +395,14 @@ struct Launch {
 
     static cudaLaunchConfig_t small_cfg(int nunits, cudaStream_t s, cudaLaunchAttribute *at)
     {
-        using C = SmallCfg<N>;
+        using C = SmallWaveCfg<N>;
+        static std::once_flag f;
+        std::call_once(f, [] {
+            cudaFuncSetAttribute(k_small_wave<N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)C::SMEM);
+            if (C::Q > 8)
+                cudaFuncSetAttribute(k_small_wave<N>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        });
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)(nunits * C::Q));
         cfg.blockDim = dim3(C::NT);
@@ -389,28 +416,15 @@ struct Launch {
         cfg.numAttrs = 1;
         return cfg;
     }
-    static void small_attrs()
-    {
-        static std::once_flag f;
-        std::call_once(f, [] {
-            using C = SmallCfg<N>;
-            cudaFuncSetAttribute(k_small_slices<N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)C::SMEM);
-            if (C::Q > 8)
-                cudaFuncSetAttribute(k_small_slices<N>,
-                                     cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        });
-    }
-    static cudaError_t small_slices(const Geom &g, int nunits, int nslices, int nsl1,
-                                    const int *slice_off, const SplatAtom *atoms, float2 *W,
-                                    float2 *T0, float2 *T1, cudaStream_t s)
+    static cudaError_t small_wave(const Geom &g, int nunits, int s0, int s1, int nsl1,
+                                  const int *slice_off, const float2 *t, float2 *W, int arbitrary,
+                                  cudaStream_t s)
     {
         if constexpr (N >= 64 && N <= 256) {
-            small_attrs();
             cudaLaunchAttribute at[1];
-            cudaLaunchConfig_t cfg = small_cfg(nunits, s, at);
-            return cudaLaunchKernelEx(&cfg, k_small_slices<N>, g, nslices, nsl1, slice_off, atoms,
-                                      W, T0, T1);
+            const cudaLaunchConfig_t cfg = small_cfg(nunits, s, at);
+            return cudaLaunchKernelEx(&cfg, k_small_wave<N>, g, nunits, s0, s1, nsl1, slice_off, t, W,
+                                      arbitrary);
         } else {
             return cudaErrorNotSupported;
         }
@@ -429,18 +443,64 @@ struct Launch {
                 init = true;
             }
             if (known[device] < 0) {
-                small_attrs();
                 cudaLaunchAttribute at[1];
                 cudaLaunchConfig_t cfg = small_cfg(1, nullptr, at);
-                int n = 0;
-                const cudaError_t e = cudaOccupancyMaxActiveClusters(&n, k_small_slices<N>, &cfg);
+                int n = 0, sms = 0;
+                cudaError_t e = cudaOccupancyMaxActiveClusters(&n, k_small_wave<N>, &cfg);
+                if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
                 if (e != cudaSuccess) cudaGetLastError();
-                known[device] = e == cudaSuccess ? n : 0;
+                known[device] = e == cudaSuccess ? std::min(n, sms / SmallWaveCfg<N>::Q) : 0;
             }
             return known[device];
         } else {
             (void)device;
             return 0;
+        }
+    }
+
+    static cudaError_t wide_wave(const Geom &g, int s0, int s1, const int *slice_off, const float2 *t,
+                                 float2 *W, int arbitrary, unsigned *count, cudaStream_t s)
+    {
+        if constexpr (WideCfg<N>::OK) {
+            using C = WideCfg<N>;
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3((unsigned)C::Q);
+            cfg.blockDim = dim3(C::NT);
+            cfg.dynamicSmemBytes = C::SMEM;
+            cfg.stream = s;
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeCooperative;  // every CTA resident at once
+            at[0].val.cooperative = 1;
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+            return cudaLaunchKernelEx(&cfg, k_wide_wave<N>, g, s0, s1, slice_off, t, W, arbitrary, count);
+        } else {
+            return cudaErrorNotSupported;
+        }
+    }
+    static bool wide_ok(int device)
+    {
+        if constexpr (WideCfg<N>::OK) {
+            static std::mutex m;
+            static int known[64];  // 1 no, 2 yes
+            if (device < 0 || device >= 64) return false;
+            std::lock_guard<std::mutex> lk(m);
+            if (!known[device]) {
+                static std::once_flag f;
+                set_smem(k_wide_wave<N>, WideCfg<N>::SMEM, f);
+                int per = 0, coop = 0, sms = 0;
+                const bool ok =
+                    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_wide_wave<N>, WideCfg<N>::NT,
+                                                                  WideCfg<N>::SMEM) == cudaSuccess &&
+                    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) == cudaSuccess &&
+                    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess;
+                if (!ok) cudaGetLastError();
+                known[device] = ok && coop && per > 0 && sms >= WideCfg<N>::Q ? 2 : 1;
+            }
+            return known[device] == 2;
+        } else {
+            (void)device;
+            return false;
         }
     }
 
@@ -454,11 +514,13 @@ struct Launch {
                                   row_plan16_ok(N) ? kRowVariants : 2, splat,
                                   splat_potential, splat_spec, col_dw, row_dwexp,
                                   col_mask, col_prop,     col_fresnel,      row_transmit_t<false>,
-                                  row_transmit_t<true>,   row_init, row_exit, row_inverse,
+                                  row_transmit_t<true>,   row_init, row_exit, row_band_inverse, row_inverse,
                                   row_intensity_t<false>, row_intensity_t<true>, row_expv,
                                   row_adj_transmit,       row_grad,         row_imgrad,
-                                  (N >= 64 && N <= 256) ? small_slices : nullptr,
-                                  (N >= 64 && N <= 256) ? small_ok : nullptr};
+                                  (N >= 64 && N <= 256) ? small_ok : nullptr,
+                                  (N >= 64 && N <= 256) ? small_wave : nullptr,
+                                  WideCfg<N>::OK ? wide_wave : nullptr,
+                                  WideCfg<N>::OK ? wide_ok : nullptr};
         return &o;
     }
 };

@@ -1003,12 +1003,14 @@ k_row_stream(const Geom g, const int *__restrict__ units, const float2 *__restri
 // MODE 0: W0 = S(wave0) * scale (start state from an incident wave; wave0
 //         shared by all units, units[i] selects the destination)
 // MODE 1: psi = iS(W) * scale, scale = 1/ny (exit wave)
-enum { kRowInit = 0, kRowExit = 1 };
+// MODE 2: iS of in-band columns (the others are not read and count as zeros),
+//         `out` may be `in`
+enum { kRowInit = 0, kRowExit = 1, kRowBand = 2 };
 
 template <int NY, int MODE>
 __global__ void __launch_bounds__(RowCfg<NY>::L * FftPlan<NY>::T)
-k_row_simple(const Geom g, const int *__restrict__ units, const float2 *__restrict__ in,
-             float2 *__restrict__ out, float scale)
+k_row_simple(const Geom g, const int *__restrict__ units, const float2 *in, float2 *out,
+             float scale)
 {
     using P = FftPlan<NY>;
     constexpr int T = P::T, E = P::E, L = RowCfg<NY>::L;
@@ -1026,8 +1028,9 @@ k_row_simple(const Geom g, const int *__restrict__ units, const float2 *__restri
     const float2 *src = (MODE == kRowInit) ? in + row : in + (size_t)u * nx * NY + row;
     float2 v[E];
 #pragma unroll
-    for (int m = 0; m < E; m++) v[m] = src[t + m * T];
-    fft_line<NY, MODE == kRowExit, 1, BLK>(v, s_lines + l * P::PADN, 0, t, g.tw_row);
+    for (int m = 0; m < E; m++)
+        v[m] = MODE == kRowBand && out_of_band(g, t + m * T) ? make_float2(0.0f, 0.0f) : src[t + m * T];
+    fft_line<NY, MODE != kRowInit, 1, BLK>(v, s_lines + l * P::PADN, 0, t, g.tw_row);
     if (row_ok) {
         float2 *dst = out + (size_t)u * nx * NY + row;
 #pragma unroll

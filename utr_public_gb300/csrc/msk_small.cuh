@@ -1,71 +1,33 @@
-// msk_small.cuh -- the whole slice loop of a small grid in one launch: one
+// msk_small.cuh -- the wave chain of a small grid's slice loop in one launch: one
 // thread-block cluster per unit (orientation x configuration).
 //
-// For N x N grids with N <= 256 a unit's buffers (the wave W = S(psi) and two
-// transmission buffers, 0.5 MB each at 256^2) stay in L2, and a slice-step is
-// too small to fill the GPU from one launch per pass: the multi-launch loop
-// spends most of its time in launch latency.  Here a cluster of Q = N/16 CTAs
-// owns one unit; CTA r owns rows [16r, 16r+16) and columns [16r, 16r+16).  Each
-// slice is two phases separated by cluster barriers (release / acquire at
-// cluster scope, so every CTA's global writes of one phase are visible to the
-// others in the next):
+// For N x N grids with N <= 256 a unit's wave W = S(psi) stays in L2, and a
+// slice-step is too small to fill the GPU from one launch per pass.  The
+// transmissions do not depend on the wave: those of a group of slices are made
+// beforehand by full launches (splat, band limit, row inverse; run_slices), t[(k -
+// s0) * nunits + u] = iS(B_k), and a cluster of Q CTAs then runs the unit's slices,
+// CTA r owning LPC rows and LPC columns:
 //
-//   row phase k:    half 0  transmit of slice k on the CTA's rows
-//                           W = S(iS(W) iS(B_k))                 (P3)
-//                   half 1  splat of slice k+1 on the same rows
-//                           A_{k+1} = S(exp(i sigma v))          (P1)
-//   column phase k: half 0  propagator of slice k on the CTA's columns
-//                           W = iF(P F(W))/nx                    (P4)
-//                   half 1  band limit of slice k+1
-//                           B_{k+1} = iF(M F(A_{k+1}))/(nx ny^2) (P2)
+//   row phase     W = S(iS(W) t_k)   on the CTA's rows (P3), t_k fetched before
+//                                    the barrier that W waits for
+//   column phase  W = iF(P F(W))/nx  on the CTA's columns (P4)
 //
-// (slices without atoms skip P1-P3).  The two CTA halves run different passes
-// at once, each with its own named barrier for its column transforms; the
-// transmissions of consecutive slices with atoms alternate between the two
-// buffers.  Every row and column is computed with the same line transforms,
-// multipliers and atom order as the multi-launch passes (k_row_splat,
-// k_col_pass, k_row_transmit), whole rows and columns instead of the in-band
-// segments.  Loads of data another CTA wrote go through L2 (ld.global.cg).
-//
-// The line transforms use the 16-points-a-thread plan (FftPlan<N, 16>: twice
-// the threads per line of the multi-launch passes, half the registers and the
-// serial chain per thread), so a CTA of 2 x 16 lines has 512 threads at 256^2;
-// the results equal the multi-launch loop's to FP32 rounding (the same
-// potentials, multipliers and atom order; another radix split of the FFT).
-// The grid is `units x Q` CTAs in clusters of Q (Q = 16 for 256^2 needs the
-// non-portable cluster size); no CTA leaves the slice loop early, so every one
-// arrives at every cluster barrier.
+// with a cluster barrier (release / acquire, so every CTA's global writes of one
+// phase are visible to the others in the next) after each, none after the columns
+// of a slice whose successor has no atoms: they stay with their CTA.  Every row and
+// column is computed with the line transforms and multipliers of the multi-launch
+// passes (k_col_pass, k_row_transmit) on the 16-points-a-thread plan
+// (FftPlan<N, 16>: twice the threads per line, half the serial chain).  Loads of
+// data another CTA wrote go through L2 (ld.global.cg).  Bound: the chain of L2
+// round trips, two transforms and a barrier of each phase.  One unit of 256^2, 32
+// slices: 0.18 ms; 0.47 ms when the other half of each CTA splatted and
+// band-limited the next slice between the same barriers -- the atom scan was the
+// longest chain of a slice.  Every CTA arrives at every cluster barrier.
 #pragma once
 
 #include "msk_passes.cuh"
 
 namespace msk {
-
-template <int N>
-struct SmallCfg {
-    static constexpr int EV = 16;  // the plan's elements per thread
-    using P = FftPlan<N, EV>;
-    static constexpr int T = P::T, E = P::E;
-    static constexpr int LPC = 16;        // rows (and columns) one CTA owns
-    static constexpr int Q = N / LPC;     // CTAs per cluster: one unit
-    static constexpr int HALF = LPC * T;  // threads of one half
-    static constexpr int NT = 2 * HALF;
-    static constexpr int RW = 32 / T;     // rows per warp in the row phase
-    static constexpr int PADN = P::PADN;
-    static constexpr int SROW = (P::PADN + 1) & ~1;
-    // shared memory in float2 units.  Row phase: half 0 a transform buffer and
-    // a stash of iS(B) per row; half 1 the splat row (potential, then the
-    // transform's exchange).  Column phase: one tile of LPC interleaved columns
-    // per half.
-    static constexpr int ROW0 = LPC * (PADN + N);
-    static constexpr int ROW1 = LPC * SROW;
-    static constexpr int COL = LPC * PADN;
-    static constexpr int F2 = (ROW0 + ROW1) > 2 * COL ? (ROW0 + ROW1) : 2 * COL;
-    static constexpr size_t SMEM = (size_t)F2 * 8 + kKnotWords * 4;
-    static_assert(N >= 64 && N <= 256, "small-grid sizes");
-    static_assert(T <= 32 && 32 % T == 0, "a warp holds whole lines");
-    static_assert(HALF % 32 == 0, "halves of whole warps");
-};
 
 __device__ __forceinline__ unsigned cluster_rank()
 {
@@ -83,117 +45,85 @@ __device__ __forceinline__ void cluster_sync()
 }
 
 template <int N>
-__global__ void __launch_bounds__(SmallCfg<N>::NT, 1)
-k_small_slices(const Geom g, int nslices, int nsl1, const int *__restrict__ slice_off,
-               const SplatAtom *__restrict__ atoms, float2 *W, float2 *Tb0, float2 *Tb1)
+struct SmallWaveCfg {
+    static constexpr int EV = 16;
+    using P = FftPlan<N, EV>;
+    static constexpr int T = P::T, E = P::E;
+    static constexpr int LPC = N >= 256 ? 16 : 8;  // rows and columns of a CTA
+    static constexpr int Q = N / LPC;
+    static constexpr int NT = LPC * T;
+    static constexpr size_t SMEM = (size_t)LPC * P::PADN * 8;
+    static_assert(NT % 32 == 0 && T <= 32, "whole warps of whole lines");
+};
+
+template <int N>
+__global__ void __launch_bounds__(SmallWaveCfg<N>::NT, 1)
+k_small_wave(const Geom g, int nunits, int s0, int s1, int nsl1, const int *__restrict__ slice_off,
+             const float2 *__restrict__ t, float2 *W, int arbitrary)
 {
-    using C = SmallCfg<N>;
-    constexpr int T = C::T, E = C::E, LPC = C::LPC, HALF = C::HALF, EV = C::EV;
+    using C = SmallWaveCfg<N>;
+    constexpr int T = C::T, E = C::E, LPC = C::LPC, EV = C::EV, PADN = C::P::PADN;
     extern __shared__ __align__(128) unsigned char smem[];
     float2 *sm = reinterpret_cast<float2 *>(smem);
-    float *s_knots = reinterpret_cast<float *>(sm + C::F2);
-
     const int rank = (int)cluster_rank();
     const int u = blockIdx.x / C::Q;
-    const int half = threadIdx.x / HALF, ht = threadIdx.x % HALF;
     const size_t plane = (size_t)N * N;
     float2 *Wu = W + (size_t)u * plane;
-    float2 *Tu[2] = {Tb0 + (size_t)u * plane, Tb1 + (size_t)u * plane};
     const int *so = slice_off + (size_t)u * nsl1;
-    for (int i = threadIdx.x; i < kKnotWords; i += C::NT) s_knots[i] = g.knots[i];
-    __syncthreads();
-
-    // row phase: line l of the CTA's rows, thread t of the line
-    const int rl = ht / T, rt = ht % T, row = rank * LPC + rl;
-    // column phase: column c of the CTA's columns, thread t of the line
-    const int cc = ht % LPC, ct = ht / LPC, col = rank * LPC + cc;
-    const float mask_scale = (1.0f / ((float)N * (float)N)) / (float)N;
-
-    // slice k's transmission lives in buffer tb[k] = (slices with atoms before k) & 1
-    int tb_next = 0;  // buffer of slice k+1, updated as the loop advances
-    int tb_cur = 0;
-    for (int k = -1; k < nslices; k++) {
-        const bool has_k = k >= 0 && so[k + 1] > so[k];
-        const bool has_n = k + 1 < nslices && so[k + 2] > so[k + 1];
-        if (k >= 0) {
-            tb_cur = tb_next;
-            tb_next = has_k ? (tb_cur ^ 1) : tb_cur;
-        }
-        // ---- row phase
-        if (half == 0) {
-            if (has_k) {  // W = S(iS(W) iS(B_k)) on this row
-                float2 *xb = sm + rl * (C::PADN + N), *stash = xb + C::PADN;
-                const float2 *brow = Tu[tb_cur] + (size_t)row * N;
-                float2 *wrow = Wu + (size_t)row * N;
-                float2 v[E];
+    const int rl = threadIdx.x / T, rt = threadIdx.x % T, row = rank * LPC + rl;
+    const int cc = threadIdx.x % LPC, ct = threadIdx.x / LPC, col = rank * LPC + cc;
+    const bool in_band = rank * LPC <= g.band_p || rank * LPC + LPC - 1 >= g.band_q;
+    float2 *wrow = Wu + (size_t)row * N;
+    float2 q[E];
+    auto fetch = [&](int k) {  // t_k on this row
+        const float2 *src = t + ((size_t)(k - s0) * nunits + u) * plane + (size_t)row * N;
 #pragma unroll
-                for (int m = 0; m < E; m++) v[m] = __ldcg(&brow[rt + m * T]);
-                fft_line<N, true, 1, 0, EV>(v, xb, 0, rt, g.tw_row16);
-#pragma unroll
-                for (int m = 0; m < E; m++) stash[rt + m * T] = v[m];
-#pragma unroll
-                for (int m = 0; m < E; m++) v[m] = __ldcg(&wrow[rt + m * T]);
-                fft_line<N, true, 1, 0, EV>(v, xb, 0, rt, g.tw_row16);
-#pragma unroll
-                for (int m = 0; m < E; m++) v[m] = cmul(v[m], stash[rt + m * T]);
-                fft_line<N, false, 1, 0, EV>(v, xb, 0, rt, g.tw_row16);
-#pragma unroll
-                for (int m = 0; m < E; m++) wrow[rt + m * T] = v[m];
-            }
-        } else if (has_n) {  // A_{k+1} = S(exp(i sigma v)) on this row
-            float2 *xb = sm + C::ROW0 + rl * C::SROW;
-            float *vacc = reinterpret_cast<float *>(xb);
-            splat_zero<N, EV>(vacc, rt);
-            __syncwarp();
-            const int wx0 = rank * LPC + ((ht >> 5) * C::RW);  // this warp's first row
-            const unsigned groups = splat_scan_warp<N, EV>(g, atoms, so[k + 1], so[k + 2], wx0, C::RW,
-                                                           row, true, rt, vacc, s_knots);
+        for (int m = 0; m < E; m++) q[m] = __ldg(&src[rt + m * T]);
+    };
+    bool has_k = so[s0 + 1] > so[s0];
+    if (has_k) fetch(s0);
+    for (int k = s0; k < s1; k++) {
+        const bool has_n = k + 1 < s1 && so[k + 2] > so[k + 1];
+        // the wave is arbitrary (not yet zero out of band) before its first
+        // propagator pass
+        const bool full = arbitrary && k == s0;
+        if (has_k) {
+            float2 *xb = sm + rl * PADN;
             float2 v[E];
-            trans_row<N, 0, EV>(g, rt, groups, vacc, xb, v);
-            float2 *arow = Tu[tb_next] + (size_t)row * N;
 #pragma unroll
             for (int m = 0; m < E; m++)
-                arow[rt + m * T] = out_of_band(g, rt + m * T) ? make_float2(0.0f, 0.0f) : v[m];
+                v[m] = band_zero<E>(m) && !full ? make_float2(0.0f, 0.0f) : __ldcg(&wrow[rt + m * T]);
+            fft_line<N, true, 1, 0, EV>(v, xb, 0, rt, g.tw_row16);
+#pragma unroll
+            for (int m = 0; m < E; m++) v[m] = cmul(v[m], q[m]);
+            fft_line<N, false, 1, 0, EV>(v, xb, 0, rt, g.tw_row16);
+#pragma unroll
+            for (int m = 0; m < E; m++)
+                if (!band_zero<E>(m) && !out_of_band(g, rt + m * T)) wrow[rt + m * T] = v[m];
         }
-        cluster_sync();
-        // ---- column phase (whole columns of the unit's grid)
-        if (half == 0) {
-            if (k >= 0) {  // W = iF(P F(W))/nx: propagator p_y then p_x, 2/3 aperture
-                float2 *buf = sm;
-                float2 v[E];
-#pragma unroll
-                for (int m = 0; m < E; m++) v[m] = __ldcg(&Wu[(size_t)(ct + m * T) * N + col]);
-                fft_line<N, false, LPC, 2, EV>(v, buf, cc, ct, g.tw_col16);
-                const int2 ab = __ldg(&g.kband[col]);
-                const float2 py = __ldg(&g.propy[col]);
-#pragma unroll
-                for (int m = 0; m < E; m++) {
-                    const int ix = ct + m * T;
-                    v[m] = (ix <= ab.x || ix >= ab.y) ? cmul(cmul(v[m], py), __ldg(&g.propx[ix]))
-                                                      : make_float2(0.0f, 0.0f);
-                }
-                fft_line<N, true, LPC, 2, EV>(v, buf, cc, ct, g.tw_col16);
-#pragma unroll
-                for (int m = 0; m < E; m++) Wu[(size_t)(ct + m * T) * N + col] = v[m];
-            }
-        } else if (has_n) {  // B_{k+1} = iF(M F(A_{k+1})) / (nx ny^2)
-            float2 *buf = sm + C::COL;
-            float2 *tu = Tu[tb_next];
+        if (has_n) fetch(k + 1);
+        if (has_k) cluster_sync();
+        if (in_band || full) {
             float2 v[E];
 #pragma unroll
-            for (int m = 0; m < E; m++) v[m] = __ldcg(&tu[(size_t)(ct + m * T) * N + col]);
-            fft_line<N, false, LPC, 2, EV>(v, buf, cc, ct, g.tw_col16);
+            for (int m = 0; m < E; m++) v[m] = __ldcg(&Wu[(size_t)(ct + m * T) * N + col]);
+            fft_line<N, false, LPC, 1, EV>(v, sm, cc, ct, g.tw_col16);
             const int2 ab = __ldg(&g.kband[col]);
+            const float2 py = __ldg(&g.propy[col]);
 #pragma unroll
             for (int m = 0; m < E; m++) {
                 const int ix = ct + m * T;
-                v[m] = (ix <= ab.x || ix >= ab.y) ? cscale(v[m], mask_scale) : make_float2(0.0f, 0.0f);
+                v[m] = !band_zero<E>(m) && (ix <= ab.x || ix >= ab.y)
+                           ? cmul(cmul(v[m], py), __ldg(&g.propx[ix]))
+                           : make_float2(0.0f, 0.0f);
             }
-            fft_line<N, true, LPC, 2, EV>(v, buf, cc, ct, g.tw_col16);
+            fft_line<N, true, LPC, 1, EV>(v, sm, cc, ct, g.tw_col16);
 #pragma unroll
-            for (int m = 0; m < E; m++) tu[(size_t)(ct + m * T) * N + col] = v[m];
+            for (int m = 0; m < E; m++) Wu[(size_t)(ct + m * T) * N + col] = v[m];
         }
-        cluster_sync();
+        if (has_n) cluster_sync();
+        else __syncthreads();  // the columns' exchange is read
+        has_k = has_n;
     }
 }
 
