@@ -424,14 +424,28 @@ Lut &lut()
 
 // ------------------------------------------------------------------ host prep
 
-// Shell sort by z (slicelib.cpp:2467-2504); same comparisons and moves, so
-// the same permutation.
-static void sort_by_z(float *x, float *y, float *z, float *occ, int *Znum, int natom)
+// The order of z as unsigned integers, -0 equal to +0.  No NaN.
+static uint32_t order_key(float z)
 {
-    int h;
-    for (h = 1; h <= (natom - 1) / 9; h = 3 * h + 1)
-        ;
-    for (; h > 0; h /= 3)
+    const float zz = z + 0.0f;
+    uint32_t u;
+    std::memcpy(&u, &zz, sizeof u);
+    return u >> 31 ? ~u : u | 0x80000000u;
+}
+
+// The Shell sort by z of slicelib.cpp:2467-2504 is passes with gaps h, the first of
+// them this one, then h / 3, to 1.
+static int first_gap(int natom)
+{
+    int h = 1;
+    while (h <= (natom - 1) / 9) h = 3 * h + 1;
+    return h;
+}
+
+// The passes as they are written there.
+static void insertion_passes(float *x, float *y, float *z, float *occ, int *Znum, int natom)
+{
+    for (int h = first_gap(natom); h > 0; h /= 3)
         for (int i = h; i < natom; i++) {
             int j = i;
             const float x2 = x[i], y2 = y[i], z2 = z[i], occ2 = occ[i];
@@ -450,6 +464,83 @@ static void sort_by_z(float *x, float *y, float *z, float *occ, int *Znum, int n
             occ[j] = occ2;
             Znum[j] = Z2;
         }
+}
+
+// The same permutation.  A pass is an insertion sort with a strict comparison of
+// each of the h interleaved subsequences, so a stable sort of each: walking the
+// atoms in order of z (equal ones in order of place), the one in place p moves to
+// place (p mod h) + h * (those of its subsequence already passed).  A radix sort by z
+// and a counting walk per pass, without the insertion loops' unpredictable
+// branches; without equal z the sorted order is the only one and needs no pass.
+// 20000 random atoms on a Grace core 0.43 ms, with the insertion loops 1.59; 2000
+// 0.025 and 0.107.  Many atoms in sets of equal z (planes of a crystal: 20000 in
+// 200 planes 1.47 and 1.24 ms), few atoms, or NaN: the insertion loops.
+static void sort_by_z(float *x, float *y, float *z, float *occ, int *Znum, int natom)
+{
+    bool plain = natom < 128;
+    for (int i = 0; i < natom && !plain; i++) plain = z[i] != z[i];
+    if (!plain) {  // a sample of them: a quarter equal to another, a few planes
+        const int m = std::min(std::max(natom / 16, 64), 1024);
+        std::vector<float> some(m);
+        for (int i = 0; i < m; i++) some[i] = z[(size_t)i * natom / m];
+        std::sort(some.begin(), some.end());
+        int equal = 0;
+        for (int i = 1; i < m; i++) equal += some[i] == some[i - 1];
+        plain = equal > m / 4;
+    }
+    if (plain) return insertion_passes(x, y, z, occ, Znum, natom);
+    struct Rec {
+        uint32_t key;
+        int atom, place;
+    };
+    const size_t n = (size_t)natom;
+    std::vector<Rec> r(n), q(n);
+    for (size_t i = 0; i < n; i++) r[i] = {order_key(z[i]), (int)i, (int)i};
+    for (int shift = 0; shift < 32; shift += 11) {
+        uint32_t start[2049] = {0};
+        for (size_t i = 0; i < n; i++) start[((r[i].key >> shift) & 2047) + 1]++;
+        for (int k = 0; k < 2048; k++) start[k + 1] += start[k];
+        for (size_t i = 0; i < n; i++) q[start[(r[i].key >> shift) & 2047]++] = r[i];
+        r.swap(q);
+    }
+    std::vector<std::pair<size_t, size_t>> ties;  // [first, last) with equal z
+    size_t crowded = 0;
+    for (size_t i = 0, j; i < n; i = j) {
+        for (j = i + 1; j < n && r[j].key == r[i].key; j++)
+            ;
+        if (j - i > 1) ties.push_back({i, j});
+        if (j - i > 16) crowded += j - i;
+    }
+    if (crowded > n / 8) return insertion_passes(x, y, z, occ, Znum, natom);
+    if (!ties.empty()) {
+        auto order_ties = [&] {
+            for (const auto &t : ties)
+                std::sort(&r[t.first], &r[0] + t.second,
+                          [](const Rec &a, const Rec &b) { return a.place < b.place; });
+        };
+        std::vector<int> passed;
+        for (int h = first_gap(natom); h > 1; h /= 3) {
+            order_ties();
+            passed.assign(h, 0);
+            // p mod h from a product: exact for p, h < 2^32 (Lemire, Kaser, Kurz,
+            // "Faster remainder by direct computation", 2019)
+            const uint64_t m = ~(uint64_t)0 / (uint64_t)h + 1;
+            for (size_t i = 0; i < n; i++) {
+                const uint64_t low = m * (uint64_t)r[i].place;
+                const int c = (int)(((unsigned __int128)low * (unsigned)h) >> 64);
+                r[i].place = c + h * passed[c]++;
+            }
+        }
+        order_ties();  // the pass with gap 1
+    }
+    std::vector<float> f(n);
+    for (float *a : {x, y, z, occ}) {
+        for (size_t i = 0; i < n; i++) f[i] = a[r[i].atom];
+        std::copy(f.begin(), f.end(), a);
+    }
+    std::vector<int> k(n);
+    for (size_t i = 0; i < n; i++) k[i] = Znum[r[i].atom];
+    std::copy(k.begin(), k.end(), Znum);
 }
 
 // Rotation about z then y' (autosliccmd.cpp:727-748), float arithmetic.
