@@ -54,19 +54,8 @@ const UtrOps *utr_ops(int n)
 namespace {
 
 constexpr double kPi = 3.14159265358979323846;
-constexpr int kScal = 10;  // per-image scalars of the gridding: sinY cosY sinZ cosZ, Fxc Fyc Fzc
 
 // ------------------------------------------------------------------ kernels
-
-struct UtrGridP {
-    int nx, ny, nz, nimg;
-    const float2 *k2;
-    const float *tabs;  // [nimg][xxx2 | xsy | xcy (nx each) | yyy2 | ysz | ycz (ny each)]
-    const float *scal;  // [nimg][kScal]
-    float fxlo, fxst, fylo, fyst, fzlo, fzst;
-    int rotshift, escc;
-    UtrAcc *acc;
-};
 
 // CT_3Dgridding (UTR.h:199-307) of every pixel of every image: the pixel's
 // frequency coordinates rotated back (about Y' then Z), on the Ewald sphere
@@ -441,12 +430,14 @@ int invlap_setup(int nx, int ny, int nz, double zaper, double yaper, double xape
 
 // Per-image coordinate tables and scalars of CT_3Dgridding (UTR.h:214-236;
 // UTR.cpp:880-898 for the angles and the centre-of-rotation factors).
-void grid_tables(const msk_utr *p, const Geo &g, int nangles, const double *angles,
-                 std::vector<float> &tabs, std::vector<float> &scal)
+// (the tables of the first ntab images: k_utr_tilt_rows reads those of one)
+void grid_tables(const msk_utr *p, const Geo &g, int nangles, int ntab, const double *angles,
+                 std::vector<float> &tabs, std::vector<float> &scal, std::vector<float> &xs)
 {
     const int nx = g.nx, ny = g.ny;
+    xs.resize(nx);
     const size_t ts = 3 * (size_t)nx + 3 * (size_t)ny;
-    tabs.resize(ts * nangles);
+    tabs.resize(ts * ntab);
     scal.resize((size_t)kScal * nangles);
     const float fxlo = (float)g.fxlo, fxst = (float)g.fxst, fylo = (float)g.fylo,
                 fyst = (float)g.fyst;
@@ -455,20 +446,23 @@ void grid_tables(const msk_utr *p, const Geo &g, int nangles, const double *angl
         const double angleZ = angles[2 * a] * pi180, angleY = angles[2 * a + 1] * pi180;
         const float sinY = (float)sin(angleY), cosY = (float)cos(angleY);
         const float sinZ = (float)sin(angleZ), cosZ = (float)cos(angleZ);
-        float *tb = tabs.data() + ts * a;
-        for (int i = 0; i < nx; i++) {
-            const float fs = fxst * (float)i;
-            const double x = (double)(fxlo + fs);
-            tb[i] = (float)(-wl2 * x * x);
-            tb[nx + i] = (float)(x * (double)sinY);
-            tb[2 * nx + i] = (float)(x * (double)cosY);
-        }
-        for (int j = 0; j < ny; j++) {
-            const float fs = fyst * (float)j;
-            const double y = (double)(fylo + fs);
-            tb[3 * nx + j] = (float)(-wl2 * y * y);
-            tb[3 * nx + ny + j] = (float)(y * (double)sinZ);
-            tb[3 * nx + 2 * ny + j] = (float)(y * (double)cosZ);
+        if (a < ntab) {
+            float *tb = tabs.data() + ts * a;
+            for (int i = 0; i < nx; i++) {
+                const float fs = fxst * (float)i;
+                const double x = (double)(fxlo + fs);
+                xs[i] = (float)x;
+                tb[i] = (float)(-wl2 * x * x);
+                tb[nx + i] = (float)(x * (double)sinY);
+                tb[2 * nx + i] = (float)(x * (double)cosY);
+            }
+            for (int j = 0; j < ny; j++) {
+                const float fs = fyst * (float)j;
+                const double y = (double)(fylo + fs);
+                tb[3 * nx + j] = (float)(-wl2 * y * y);
+                tb[3 * nx + ny + j] = (float)(y * (double)sinZ);
+                tb[3 * nx + 2 * ny + j] = (float)(y * (double)cosZ);
+            }
         }
         const double cy = cos(angleY), sy = sin(angleY), cz = cos(angleZ), sz = sin(angleZ);
         const float ax = (float)(tpi * (p->dxc * (1.0 - cy * cz) - p->dyc * sz + p->dzc * sy * cz));
@@ -628,8 +622,8 @@ int spectra(msk_context *ctx, const msk_utr *p, int a0, int nangles, const float
     return MSK_OK;
 }
 
-int grid_launch(msk_context *ctx, const msk_utr *p, const Geo &g, int nangles, const float2 *k2,
-                const float *tabs_d, const float *scal_d, UtrAcc *acc)
+UtrGridP grid_params(const msk_utr *p, const Geo &g, int nangles, const float2 *k2,
+                     const float *tabs_d, const float *scal_d, UtrAcc *acc)
 {
     UtrGridP gp{};
     gp.nx = g.nx;
@@ -645,9 +639,17 @@ int grid_launch(msk_context *ctx, const msk_utr *p, const Geo &g, int nangles, c
     gp.fyst = (float)g.fyst;
     gp.fzlo = (float)g.fzlo;
     gp.fzst = (float)g.fzst;
+    gp.wl2 = (float)(0.5 * p->wl);
     gp.rotshift = p->dxc != 0 || p->dyc != 0 || p->dzc != 0;
     gp.escc = p->escc != 0;
     gp.acc = acc;
+    return gp;
+}
+
+int grid_launch(msk_context *ctx, const msk_utr *p, const Geo &g, int nangles, const float2 *k2,
+                const float *tabs_d, const float *scal_d, UtrAcc *acc)
+{
+    const UtrGridP gp = grid_params(p, g, nangles, k2, tabs_d, scal_d, acc);
     const size_t n = (size_t)g.nx * g.ny * nangles;
     Prof pr(ctx, kUtrGrid, 8.0 * n);
     k_utr_grid<<<grid_blocks(n), 256, 0, ctx->stream>>>(gp);
@@ -770,9 +772,18 @@ int msk_utr_reconstruct_planes(msk_context *ctx, const msk_utr *p, int nangles,
             : p->asigma * p->wl / (4.0 * kPi * sqrt(1.0 + p->asigma * p->asigma) * g.xst);
 
     // tables
-    std::vector<float> tabs, scal;
-    grid_tables(p, g, nangles, angles, tabs, scal);
-    std::vector<float2> twx, twy, twz;
+    std::vector<float2> twx, twy, twz, twx16;
+    // orientations about y alone: one pass from the spectra to the Fourier rows,
+    // for rows of 256 to 1024 points and two CTAs an SM at least.  256^3 from 31
+    // images 0.39 ms (general path 0.57), 512^3 from 31 1.90 (3.19), from 600 6.7
+    // (14.9), 1024^2 x 128 from 90 5.4 (5.4); shorter rows leave too few CTAs, each
+    // with all images: 64^3 from 180 0.35 (0.21), 128^3 from 90 0.24 (0.24)
+    const UtrOps *xop = utr_ops(nx);
+    bool tilt = xop->tilt_rows && (size_t)ny * ((nz + xop->tilt_k - 1) / xop->tilt_k) >= 2 * 152 &&
+                std::isfinite(p->wl) && twiddles(nx, twx16, 16);
+    for (int a = 0; a < nangles; a++) tilt = tilt && angles[2 * a] == 0.0 && std::isfinite(angles[2 * a + 1]);
+    std::vector<float> tabs, scal, xs;
+    grid_tables(p, g, nangles, tilt ? 1 : nangles, angles, tabs, scal, xs);
     if (!twiddles(nx, twx) || !twiddles(ny, twy) || !twiddles(nz, twz))
         return fail(ctx, MSK_EUNSUPPORTED, "no FFT for this size");
     // input image planes (UTR.cpp:920-940): per image the operation, cos and
@@ -796,6 +807,7 @@ int msk_utr_reconstruct_planes(msk_context *ctx, const msk_utr *p, int nangles,
     const size_t o_pop = pk.put(pop), o_ppar = pk.put(ppar);
     std::vector<float> fill0(nangles, 0.0f);
     const size_t o_fill = pk.put(fill0);
+    const size_t o_twx16 = pk.put(twx16), o_xs = pk.put(xs);
     const size_t o_twx = pk.put(twx), o_twy = pk.put(twy), o_twz = pk.put(twz);
     const CorrOffsets oc = put_corr(pk, ct, nx, ny, nz);
     const size_t o_mx = pk.put(mx), o_my = pk.put(my), o_mz = pk.put(mz);
@@ -812,9 +824,12 @@ int msk_utr_reconstruct_planes(msk_context *ctx, const msk_utr *p, int nangles,
     Geom gflags{};  // the call's device error flag, cleared once
     if ((st = flags_reset(ctx, gflags))) return st;
     MSK_CUDA(ctx, ctx->utr_k2.reserve(sizeof(float2) * plane * nangles));
-    MSK_CUDA(ctx, ctx->utr_acc.reserve(sizeof(UtrAcc) * nvox));
-    UtrAcc *acc = ctx->utr_acc.as<UtrAcc>();
-    MSK_CUDA(ctx, cudaMemsetAsync(acc, 0, sizeof(UtrAcc) * nvox, ctx->stream));
+    UtrAcc *acc = nullptr;
+    if (!tilt) {
+        MSK_CUDA(ctx, ctx->utr_acc.reserve(sizeof(UtrAcc) * nvox));
+        acc = ctx->utr_acc.as<UtrAcc>();
+        MSK_CUDA(ctx, cudaMemsetAsync(acc, 0, sizeof(UtrAcc) * nvox, ctx->stream));
+    }
     const float *tabs_d = reinterpret_cast<const float *>(tb + o_tabs);
     const float *scal_d = reinterpret_cast<const float *>(tb + o_scal);
     const int tstride = 3 * nx + 3 * ny;
@@ -844,7 +859,8 @@ int msk_utr_reconstruct_planes(msk_context *ctx, const msk_utr *p, int nangles,
             MSK_CUDA(ctx, cudaEventRecord(ev, ctx->aux));
             MSK_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ev, 0));
             if ((st = spectra(ctx, p, a0, na, dst, tw_x, tw_y, gflags.err))) return st;
-            if ((st = grid_launch(ctx, p, g, na, ctx->utr_k2.as<float2>() + (size_t)a0 * plane,
+            if (!tilt &&
+                (st = grid_launch(ctx, p, g, na, ctx->utr_k2.as<float2>() + (size_t)a0 * plane,
                                   tabs_d + (size_t)a0 * tstride, scal_d + (size_t)a0 * kScal,
                                   acc)))
                 return st;
@@ -882,14 +898,20 @@ int msk_utr_reconstruct_planes(msk_context *ctx, const msk_utr *p, int nangles,
         } else if ((st = spectra(ctx, p, 0, nangles, img_d, tw_x, tw_y, gflags.err))) {
             return st;
         }
-        if ((st = grid_launch(ctx, p, g, nangles, ctx->utr_k2.as<float2>(), tabs_d, scal_d, acc)))
+        if (!tilt &&
+            (st = grid_launch(ctx, p, g, nangles, ctx->utr_k2.as<float2>(), tabs_d, scal_d, acc)))
             return st;
     }
 
     // Fourier-space processing and the inverse 3D transform
     MSK_CUDA(ctx, ctx->utr_vol.reserve(sizeof(float2) * nvox));
     float2 *vol = ctx->utr_vol.as<float2>();
-    {
+    if (tilt) {
+        Prof pr(ctx, kUtrFourier, 8.0 * (nvox + plane * nangles));
+        UtrGridP gp = grid_params(p, g, nangles, ctx->utr_k2.as<float2>(), tabs_d, scal_d, nullptr);
+        gp.xs = reinterpret_cast<const float *>(tb + o_xs);
+        utr_ops(nx)->tilt_rows(gp, fr, reinterpret_cast<const float2 *>(tb + o_twx16), vol, ctx->stream);
+    } else {
         Prof pr(ctx, kUtrFourier, 24.0 * nvox);
         utr_ops(nx)->fourier_rows(fr, tw_x, acc, vol, ny * nz, ctx->stream);
     }
@@ -982,8 +1004,8 @@ int msk_utr_grid(msk_context *ctx, const msk_utr *p, int nangles, const double *
     if (st) return st;
     if (g.nx < 2 || g.ny < 2 || g.nz < 2) return fail(ctx, MSK_EINVAL, "volume too small");
     MSK_CUDA(ctx, cudaSetDevice(ctx->device));
-    std::vector<float> tabs, scal;
-    grid_tables(p, g, nangles, angles, tabs, scal);
+    std::vector<float> tabs, scal, xs;
+    grid_tables(p, g, nangles, nangles, angles, tabs, scal, xs);
     TabPack pk;
     const size_t o_tabs = pk.put(tabs), o_scal = pk.put(scal);
     unsigned char *tb = upload_pack(ctx, pk, &st);

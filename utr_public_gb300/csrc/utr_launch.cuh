@@ -18,6 +18,12 @@ struct UtrOps {
     // rows of the volume (x lines of length n): gridding sums -> inverse FFT
     void (*fourier_rows)(const UtrFourier &, const float2 *tw, const UtrAcc *acc, float2 *vol,
                          int nrows, cudaStream_t);
+    // gridding and fourier_rows in one pass, for orientations about y alone (tw16:
+    // the 16-points-a-thread plan's twiddles); null for other lengths.  A CTA has
+    // tilt_k rows of consecutive z.
+    int tilt_k;
+    void (*tilt_rows)(const UtrGridP &, const UtrFourier &, const float2 *tw16, float2 *vol,
+                      cudaStream_t);
     // column passes over lines of length n (units x width columns of a 2D view)
     void (*col_img)(const UtrCol &, const CUtensorMap &in, const CUtensorMap &out, int units,
                     cudaStream_t);
@@ -44,6 +50,17 @@ template <int N> struct UtrLaunch {
         set_smem(k_utr_fourier_rows<N>, Smem<N>::row, f);
         const int L = RowCfg<N>::L;
         k_utr_fourier_rows<N><<<(nrows + L - 1) / L, L * P::T, Smem<N>::row, s>>>(fr, tw, acc, vol);
+    }
+    static void tilt_rows(const UtrGridP &p, const UtrFourier &fr, const float2 *tw16, float2 *vol,
+                          cudaStream_t s)
+    {
+        if constexpr (UtrTiltCfg<N>::OK) {
+            using C = UtrTiltCfg<N>;
+            static std::once_flag f;
+            set_smem(k_utr_tilt_rows<N>, C::SMEM, f);
+            const int kb = (p.nz + C::K - 1) / C::K;
+            k_utr_tilt_rows<N><<<(unsigned)(p.ny * kb), C::NT, C::SMEM, s>>>(p, fr, tw16, vol);
+        }
     }
     template <int MODE>
     static void col(const UtrCol &p, const CUtensorMap &in, const CUtensorMap &out, int units,
@@ -73,7 +90,8 @@ template <int N> struct UtrLaunch {
     {
         static const UtrOps o = {N,       UtrColCfg<N>::C, UtrColCfg<N>::BR, UtrColCfg<N, true>::C,
                                  img_rows,
-                                 fourier_rows, col_img, col_vol, col_final};
+                                 fourier_rows, UtrTiltCfg<N>::K, UtrTiltCfg<N>::OK ? tilt_rows : nullptr,
+                                 col_img, col_vol, col_final};
         return &o;
     }
 };
