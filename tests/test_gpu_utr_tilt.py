@@ -1,6 +1,6 @@
 """Reconstruction from orientations about y alone (gridding and Fourier rows in one
-pass, rows of 256 to 1024 points and enough of them; the others take the general
-path both times) against the general path: a rotation of 360
+pass, rows of 256 to 1024 points, enough of them and a depth of half the width or
+more; the others take the general path both times) against the general path: a rotation of 360
 degrees about z for the first orientation leaves every coordinate as it is
 (sin is 2e-16 there) but is not an orientation about y alone.
 
@@ -28,7 +28,8 @@ ANGLES = {1: [0.0], 2: [90.0, 0.02], 31: np.linspace(0.0, 174.0, 31), 40: np.lin
     (256, 16, 128, 31, {}), (512, 16, 512, 40, {"nsr": 0.02}), (512, 32, 16, 2, {}),
     (1024, 16, 256, 31, {"dyc": 0.4}), (256, 64, 256, 1, {}), (32, 32, 32, 31, {}), (2048, 16, 16, 2, {}),
     (256, 128, 128, 31, {}), (512, 512, 16, 2, {}), (256, 512, 16, 40, {}),
-    (512, 64, 256, 40, {"dxc": 1.3, "dzc": -0.7})])
+    (512, 64, 256, 40, {"dxc": 1.3, "dzc": -0.7}), (1024, 16, 512, 31, {"dyc": 0.4}),
+    (256, 16, 1024, 40, {})])
 def test_tilt_rows(ctx, msk, nx, ny, nz, n, kw, escc):
     p = params(nx, ny, nz, escc=escc, **kw)
     im = images(p, n, seed=nx + nz)

@@ -774,13 +774,17 @@ int msk_utr_reconstruct_planes(msk_context *ctx, const msk_utr *p, int nangles,
     // tables
     std::vector<float2> twx, twy, twz, twx16;
     // orientations about y alone: one pass from the spectra to the Fourier rows,
-    // for rows of 256 to 1024 points and two CTAs an SM at least.  256^3 from 31
-    // images 0.39 ms (general path 0.57), 512^3 from 31 1.90 (3.19), from 600 6.7
-    // (14.9), 1024^2 x 128 from 90 5.4 (5.4); shorter rows leave too few CTAs, each
-    // with all images: 64^3 from 180 0.35 (0.21), 128^3 from 90 0.24 (0.24)
+    // for rows of 256 to 1024 points, two CTAs an SM at least and a depth of half
+    // the width or more.  256^3 from 31 images 0.39 ms (general path 0.57), 512^3
+    // from 31 1.90 (3.19), from 600 6.7 (14.9), 512^2 x 256 from 180 2.55 (3.64),
+    // 1024^3 from 180 20.6 (35.0).  Shorter rows leave too few CTAs, each with all
+    // images: 64^3 from 180 0.35 (0.21); in a flat volume neighbouring pixels fall
+    // into one voxel and their adds wait for one another: 1024^2 x 128 from 90 5.4
+    // (5.4), from host images 10.1 (9.0), whose copy the general path's gridding
+    // runs beside
     const UtrOps *xop = utr_ops(nx);
     bool tilt = xop->tilt_rows && (size_t)ny * ((nz + xop->tilt_k - 1) / xop->tilt_k) >= 2 * 152 &&
-                std::isfinite(p->wl) && twiddles(nx, twx16, 16);
+                2 * nz >= nx && std::isfinite(p->wl) && twiddles(nx, twx16, 16);
     for (int a = 0; a < nangles; a++) tilt = tilt && angles[2 * a] == 0.0 && std::isfinite(angles[2 * a + 1]);
     std::vector<float> tabs, scal, xs;
     grid_tables(p, g, nangles, tilt ? 1 : nangles, angles, tabs, scal, xs);
