@@ -3655,7 +3655,7 @@ extern "C" int msk_tilt_series_batch(msk_context *ctx, const msk_series *s, int 
     size_t free_b = 0, total_b = 0;
     MSK_CUDA(ctx, cudaMemGetInfo(&free_b, &total_b));
     const size_t budget = (size_t)((double)(free_b + ctx->arena.cap) * 0.8);
-    auto arena_of = [&](SpecPlan &q, size_t &up, size_t &work) {
+    auto arena_of = [&](SpecPlan &q, size_t &up, size_t &work, bool groups) {
         const size_t plane = (size_t)q.gp.nx * q.gp.ny;
         q.o_tab = up;
         up += align256(q.tables.size());
@@ -3665,8 +3665,13 @@ extern "C" int msk_tilt_series_batch(msk_context *ctx, const msk_series *s, int 
         up += align256(q.b.slice_off.size() * sizeof(int));
         q.o_act = up;
         q.small = small_grid_ok(ctx, q.gp, s->nmode, q.nunits);
-        q.group = group_size(plane, q.nunits, q.nslices, s->nmode, kGroupPoints / plane);
-        if (q.group > 1 && q.b.gstart.empty()) group_slices(q.b, q.group);
+        q.group = groups ? group_size(plane, q.nunits, q.nslices, s->nmode, kGroupPoints / plane) : 1;
+        if (q.group <= 1) {
+            q.b.gstart.clear();
+            q.b.actv.clear();
+        } else if (q.b.gstart.empty()) {
+            group_slices(q.b, q.group);
+        }
         const size_t grids = (size_t)q.nunits * q.group;
         up += align256(std::max<size_t>(q.b.act.size() + q.b.actv.size(), 1) * sizeof(int));
         q.o_meta = up;
@@ -3703,8 +3708,12 @@ extern "C" int msk_tilt_series_batch(msk_context *ctx, const msk_series *s, int 
         size_t up = 0, work = 0;
         for (; last < nspec; last++) {
             size_t up2 = up, work2 = work;
-            arena_of(P[last], up2, work2);
+            arena_of(P[last], up2, work2, true);
             if (last > first && up2 + work2 > budget) break;
+            if (up2 + work2 > budget) {  // alone and short of memory: a slice at a time
+                up2 = up, work2 = work;
+                arena_of(P[last], up2, work2, false);
+            }
             up = up2;
             work = work2;
         }
