@@ -1,5 +1,6 @@
 """The wave chain of small calls in one launch per slice group: clusters for grids of
-64^2 to 256^2, one cooperative launch for a lone unit of 512^2 or 1024^2.
+64^2 to 256^2 (more CTAs than SMs, too), one cooperative launch for a lone unit of
+512^2 or 1024^2.
 MSK_SMALL_GRID=0 selects the launch-per-pass loop, whose 32-point plans the wide
 kernel shares (the same bits); the cluster kernel's plan is another (relative L2
 2e-6), and both are within 1e-5 of the FP64 oracle.  An incident wave of white noise
@@ -61,7 +62,8 @@ def test_calculate(ctx, msk, oracle, n, dz, wave):
 
 
 @pytest.mark.parametrize("dw", [False, True])
-@pytest.mark.parametrize("n,na", [(64, 1), (64, 7), (128, 3), (256, 5), (512, 1), (1024, 1)])
+@pytest.mark.parametrize("n,na", [(64, 1), (64, 7), (64, 200), (128, 3), (128, 19), (256, 5), (512, 1),
+                                  (1024, 1)])
 def test_tilt_series(ctx, msk, n, na, dw):
     at = atoms_with_gaps(n)
     s = msk.Series()

@@ -1698,11 +1698,13 @@ static int reserve_transmissions(msk_context *ctx, size_t plane, size_t units, s
 // (k_small_wave, msk_small.cuh), one per slice group: square grids of 64^2 to
 // 256^2, on a device that fits the clusters.  MSK_SMALL_GRID=0 in the environment
 // keeps the launch-per-pass loop (=1: the default).
-// Only when the units' clusters have an SM a CTA each: with more, the loop keeps
-// the whole GPU busy and is faster (64 orientations of a 256^2 specimen in
-// clusters 116k slice-steps/s against 188k in the loop), while a few units leave
-// the loop's launches latency-bound (one unit of 256^2, 32 slices: 0.18 ms
-// against ~0.5).
+// Up to a number of units (SmallWaveCfg::PER CTAs an SM), as few leave the loop's
+// launches latency-bound and many keep the whole GPU busy in the loop.  Tilt series,
+// loop / clusters in ms: 256^2 10 units 2.66 / 2.48, 18 units 3.72 / 3.75, 45 units
+// 4.57 / 6.15; 128^2 10 units 2.11 / 1.68, 24 units 2.86 / 2.48, 45 units 3.16 / 3.12; 64^2
+// 30 units 2.82 / 2.28, 120 units 4.40 / 3.63, 240 units 6.15 / 5.99.  Batches fill the
+// GPU sooner: 12 specimens of 20 units of 128^2 7.44 / 6.80, 16 of 36 12.8 / 13.6, 8 of
+// 150 units of 64^2 10.1 / 9.3.
 static bool small_grid_ok(msk_context *ctx, const GridPre &gp, int nmode, int nunits)
 {
     const char *forced = getenv("MSK_SMALL_GRID");

@@ -97,8 +97,8 @@ struct SizeOps {
     // returns the number of loss partials written
     int (*row_imgrad)(const Geom &, int nunits, const float2 *E, const float *target,
                       size_t tstride, float2 *G, double *partial, cudaStream_t);
-    // square grids of 64 <= N <= 256 (null for other sizes).  small_ok: how many
-    // units' clusters the device runs at once, an SM a CTA (0: none fit)
+    // square grids of 64 <= N <= 256 (null for other sizes).  small_ok: up to
+    // how many units the clusters are the faster way (0: none fit the device)
     int (*small_ok)(int device);
     // the wave chain of slices s0 .. s1-1 alone, from transmissions iS(B) made
     // beforehand (grid (k - s0) * nunits + u of t); arbitrary: W may hold anything
@@ -449,7 +449,8 @@ struct Launch {
                 cudaError_t e = cudaOccupancyMaxActiveClusters(&n, k_small_wave<N>, &cfg);
                 if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
                 if (e != cudaSuccess) cudaGetLastError();
-                known[device] = e == cudaSuccess ? std::min(n, sms / SmallWaveCfg<N>::Q) : 0;
+                known[device] =
+                    e == cudaSuccess && n > 0 ? sms * SmallWaveCfg<N>::PER / SmallWaveCfg<N>::Q : 0;
             }
             return known[device];
         } else {

@@ -51,6 +51,8 @@ struct SmallWaveCfg {
     static constexpr int T = P::T, E = P::E;
     static constexpr int LPC = N >= 256 ? 16 : 8;  // rows and columns of a CTA
     static constexpr int Q = N / LPC;
+    // CTAs an SM up to which a call's clusters beat the launch loop (small_grid_ok)
+    static constexpr int PER = N >= 256 ? 1 : N >= 128 ? 2 : 8;
     static constexpr int NT = LPC * T;
     static constexpr size_t SMEM = (size_t)LPC * P::PADN * 8;
     static_assert(NT % 32 == 0 && T <= 32, "whole warps of whole lines");
