@@ -2383,6 +2383,13 @@ int tilt_series_impl(msk_context *ctx, const msk_series *s, int natom, const int
         if (st) return st;
         b.call_units = nunits;
         float2 *psi = ctx->psi.as<float2>(), *tb = ctx->tbuf.as<float2>();
+        if (bi > 0 && (spherical || s->nmode != 0)) {
+            // transmits of whole rows (nmode 1 and 2, the first slice of a spherical
+            // wave) read the transmissions' out-of-band columns: zeros again where the
+            // exit waves and image planes of the batch before were
+            for (DevBuf *t : {&ctx->tbuf, &ctx->tbuf2})
+                MSK_CUDA(ctx, cudaMemsetAsync(t->p, 0, (size_t)nb * plane * sizeof(float2), ctx->stream));
+        }
         if (spherical) {
             Prof p(ctx, kInit, 8.0 * plane * (nb + 1));
             rop->row_init(gp.g, nullptr, nb, ctx->wave0.as<float2>(), psi, 1.0f, ctx->stream);
