@@ -1657,41 +1657,41 @@ static int group_size(size_t plane, int nunits, int nslices, int nmode, size_t g
     return (int)std::max<size_t>(1, std::min<size_t>(want, nslices));
 }
 
-// The slice loop over a batch: the psi buffer holds W0 = S(wave0) on entry
-// and W = S(exit wave) on return.
-//
-// Two chains per slice: the transmission chain (P1 splat, P2 band limit) and
-// the wave chain (P3 transmit, P4 propagate).  With two transmission buffers
-// the transmission chain of the next non-empty slice runs on the context's
-// stream while the wave chain of the current one runs on the second stream,
-// so the compute-bound splat overlaps the memory-bound wave passes.  Events
-// order P3 after its P2 and the reuse of a transmission buffer after the P3
-// that read it.  The transmissions do not depend on the wave: with few units in
-// the batch those of a group of slices (Batch::gstart) are made in one launch
-// per pass, so that the chain runs at the rate of full launches instead of one
-// launch's latency per slice.  With per-kernel profiling on, everything runs in order on
-// one stream so that each launch is timed alone.
 // The transmission buffers (two sets, and the Debye-Waller branch's spectra) of
 // `grids` grids each; `grids` becomes `units`, one per unit and no groups, where
-// the device has no memory for more.
+// groups would take over half of the free memory, or the device has none for them.
 static int reserve_transmissions(msk_context *ctx, size_t plane, size_t units, size_t &grids, bool spec)
 {
-    for (;;) {
-        cudaError_t e = ctx->tbuf.reserve(grids * plane * sizeof(float2));
-        if (e == cudaSuccess) e = ctx->tbuf2.reserve(ctx->tbuf.cap);
-        if (e == cudaSuccess && spec) e = ctx->spec.reserve(ctx->tbuf.cap);
+    const std::vector<DevBuf *> bufs = spec ? std::vector<DevBuf *>{&ctx->tbuf, &ctx->tbuf2, &ctx->spec}
+                                            : std::vector<DevBuf *>{&ctx->tbuf, &ctx->tbuf2};
+    auto bytes = [&] { return grids * plane * sizeof(float2); };
+    if (grids > units) {
+        size_t grow = 0, free_b = 0, total_b = 0;
+        for (DevBuf *b : bufs) grow += bytes() - std::min(bytes(), b->cap);
+        if (grow) MSK_CUDA(ctx, cudaMemGetInfo(&free_b, &total_b));
+        if (grow > free_b / 2) grids = units;
+    }
+    for (bool again = false;; again = true) {
+        cudaError_t e = cudaSuccess;
+        for (DevBuf *b : bufs)
+            if (e == cudaSuccess) e = b->reserve(bytes());
         ctx->group_grids = grids;
         if (e == cudaSuccess) return MSK_OK;
-        if (e != cudaErrorMemoryAllocation || grids <= units) {
+        if (e != cudaErrorMemoryAllocation || again) {
             MSK_CUDA(ctx, e);
             return MSK_ECUDA;
         }
-        cudaGetLastError();  // not sticky: fewer grids
-        ctx->tbuf.release();
-        ctx->tbuf2.release();
-        ctx->spec.release();
+        cudaGetLastError();  // not sticky: without groups, and without what larger calls left
+        for (DevBuf *b : {&ctx->tbuf, &ctx->tbuf2, &ctx->spec}) b->release();
         grids = units;
     }
+}
+
+// Bytes of each of the call's transmission buffers (a buffer may be larger: it keeps
+// the size of the largest call).
+static size_t transmission_bytes(const msk_context *ctx, const GridPre &gp)
+{
+    return std::max(ctx->units_alloc, ctx->group_grids) * gp.nx * gp.ny * sizeof(float2);
 }
 
 // Whether the wave chain of this grid's slice loop runs as cluster launches
@@ -1715,7 +1715,7 @@ static bool small_grid_ok(msk_context *ctx, const GridPre &gp, int nmode, int nu
 
 static bool small_path(msk_context *ctx, const GridPre &gp, const Batch &b, int nmode)
 {
-    return ctx->tbuf2.cap >= ctx->tbuf.cap && ctx->tbuf.cap > 0 &&
+    return ctx->tbuf2.cap >= transmission_bytes(ctx, gp) &&
            small_grid_ok(ctx, gp, nmode, std::max(b.nunits, b.call_units));
 }
 
@@ -1727,18 +1727,33 @@ static bool wide_path(msk_context *ctx, const GridPre &gp, const Batch &b, int n
     if (forced && forced[0] == '0') return false;
     const SizeOps *op = size_ops(gp.nx);
     return nmode == 0 && gp.nx == gp.ny && op && op->wide_wave && b.nunits == 1 && b.call_units <= 1 &&
-           ctx->tbuf2.cap >= ctx->tbuf.cap && ctx->tbuf.cap > 0 && op->wide_ok(ctx->device);
+           ctx->tbuf2.cap >= transmission_bytes(ctx, gp) && op->wide_ok(ctx->device);
 }
 
+// The slice loop over a batch: the psi buffer holds W0 = S(wave0) on entry
+// and W = S(exit wave) on return.
+//
+// Two chains per slice: the transmission chain (P1 splat, P2 band limit) and
+// the wave chain (P3 transmit, P4 propagate).  With two transmission buffers
+// the transmission chain of the next non-empty slice runs on the context's
+// stream while the wave chain of the current one runs on the second stream,
+// so the compute-bound splat overlaps the memory-bound wave passes.  Events
+// order P3 after its P2 and the reuse of a transmission buffer after the P3
+// that read it.  The transmissions do not depend on the wave: with few units in
+// the batch those of a group of slices (Batch::gstart) are made in one launch
+// per pass, so that the chain runs at the rate of full launches instead of one
+// launch's latency per slice.  With per-kernel profiling on, everything runs in order on
+// one stream so that each launch is timed alone.
 int run_slices(msk_context *ctx, const GridPre &gp, const Batch &b, int nmode, bool w_in_band)
 {
     const SizeOps *rop = size_ops(gp.ny), *cop = size_ops(gp.nx);
     const Geom &g = gp.g;
     const bool small = small_path(ctx, gp, b, nmode), wide = wide_path(ctx, gp, b, nmode);
     const bool dw = !b.dw.empty();
-    if (dw && ctx->spec.cap < ctx->tbuf.cap)
+    const size_t tbytes = transmission_bytes(ctx, gp);
+    if (dw && ctx->spec.cap < tbytes)
         return fail(ctx, MSK_EUNSUPPORTED, "the Debye-Waller branch needs a buffer of its own");
-    const bool overlap = !ctx->prof_on && ctx->tbuf2.cap >= ctx->tbuf.cap;
+    const bool overlap = !ctx->prof_on && ctx->tbuf2.cap >= tbytes;
     // launches of the wave chain that do not fill the GPU go first, ahead of the
     // transmissions of later slices, which have slack (45 units of 256^2 6.5 -> 6.1
     // ms, one of 1024^2 5.99 -> 5.75); large ones do not (16 of 1024^2: 33.8 -> 34.4)
@@ -2239,8 +2254,10 @@ int tilt_series_impl(msk_context *ctx, const msk_series *s, int natom, const int
     const size_t img_bytes = (size_t)ndefocus * plane * sizeof(float);
     size_t budget = free_b - std::min(free_b, (size_t)(img_direct ? 0 : img_bytes));
     budget = std::min<size_t>(budget / 2, (size_t)64 << 30);
-    // psi and two transmission buffers per unit in flight
-    int B = (int)std::max<size_t>(1, std::min<size_t>(nunits, budget / (3 * plane * sizeof(float2))));
+    // psi, two transmission buffers and (Debye-Waller) the spectra per unit in flight
+    const bool dw_branch = s->lwobble && nconfig == 1;
+    const size_t planes = dw_branch ? 4 : 3;
+    int B = (int)std::max<size_t>(1, std::min<size_t>(nunits, budget / (planes * plane * sizeof(float2))));
     if (s->max_batch > 0) B = std::min(B, s->max_batch);
     if (nconfig > 1 && B > nconfig) B = (B / nconfig) * nconfig;  // whole angles per batch
     // batch bounds: a large call starts with a small batch (~1/16 of the
@@ -2294,8 +2311,8 @@ int tilt_series_impl(msk_context *ctx, const msk_series *s, int natom, const int
         ev_copied = ctx->stk_ev[1];
     }
     // grids per transmission buffer: one per unit, or a group of slices of them
-    const bool dw_branch = s->lwobble && nconfig == 1;
-    size_t grids = std::max<size_t>(B, std::min<size_t>(kGroupPoints / plane, (size_t)B * nslices));
+    const size_t in_group = s->nmode == 0 ? std::min<size_t>(kGroupPoints / plane, (size_t)B * nslices) : 1;
+    size_t grids = std::max<size_t>(B, in_group);
     MSK_CUDA(ctx, ctx->psi.reserve((size_t)B * plane * sizeof(float2)));
     if ((st = reserve_transmissions(ctx, plane, B, grids, dw_branch))) return st;
     // the splat stores in-band row segments only: the rest must read as zeros
