@@ -1719,8 +1719,10 @@ static bool small_path(msk_context *ctx, const GridPre &gp, const Batch &b, int 
            small_grid_ok(ctx, gp, nmode, std::max(b.nunits, b.call_units));
 }
 
-// The same for a lone unit of 512^2 or 1024^2 (k_wide_wave): it computes what the
-// launch loop's 32-point plans compute.  MSK_SMALL_GRID=0 keeps the loop here too.
+// The same for a lone unit of 512^2 or 1024^2 (k_wide_wave), where the propagator's and
+// the transmit's schedules are 32-point plans (run_slices): it computes what those
+// compute, so that a unit alone gives the bits it gives among several.
+// MSK_SMALL_GRID=0 keeps the loop here too.
 static bool wide_path(msk_context *ctx, const GridPre &gp, const Batch &b, int nmode)
 {
     const char *forced = getenv("MSK_SMALL_GRID");
@@ -1748,7 +1750,7 @@ int run_slices(msk_context *ctx, const GridPre &gp, const Batch &b, int nmode, b
 {
     const SizeOps *rop = size_ops(gp.ny), *cop = size_ops(gp.nx);
     const Geom &g = gp.g;
-    const bool small = small_path(ctx, gp, b, nmode), wide = wide_path(ctx, gp, b, nmode);
+    const bool small = small_path(ctx, gp, b, nmode);
     const bool dw = !b.dw.empty();
     const size_t tbytes = transmission_bytes(ctx, gp);
     if (dw && ctx->spec.cap < tbytes)
@@ -1773,9 +1775,10 @@ int run_slices(msk_context *ctx, const GridPre &gp, const Batch &b, int nmode, b
     if (grouped) gg.group_units = b.nunits;
     const size_t grids = std::max(ctx->units_alloc, ctx->group_grids);
     ColView tmaps[2], pmap;
-    // (the wave chain of a small grid or a lone unit runs without these plans)
-    const int vm = col_variant(ctx, gp, kColMask), vp = small || wide ? 0 : col_variant(ctx, gp, kColProp);
-    const int rv = small || wide ? 0 : row_variant(ctx, gp);
+    // (the wave chain of a small grid runs without the last two)
+    const int vm = col_variant(ctx, gp, kColMask), vp = small ? 0 : col_variant(ctx, gp, kColProp);
+    const int rv = small ? 0 : row_variant(ctx, gp);
+    const bool wide = wide_path(ctx, gp, b, nmode) && vp < 2 && rv < 2;
     int st = column_map(ctx, &tmaps[0], tbs[0], gp.nx, gp.ny, grids, cop, vm);
     if (st) return st;
     st = column_map(ctx, &tmaps[1], tbs[1], gp.nx, gp.ny, grids, cop, vm);
