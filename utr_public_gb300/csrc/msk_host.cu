@@ -1114,24 +1114,26 @@ void prof_collect(msk_context *ctx)
 
 namespace {
 
-// Times launch(v) for the variants v in [0, nv): two warm-up launches of every
+// Times launch(v) for the variants v in [0, nv): a warm-up launch of every
 // variant, then kTuneRounds rounds in which every variant runs between two
 // events, the order rotating from round to round; ms[v] = the variant's fastest
 // run.  Interleaving the variants keeps a clock that is still rising (the
 // first launches of a process) from favouring whichever variant runs last.  A
 // run is as many launches back to back as take about kTuneMs: the event clock
 // moves in steps of 2 us, as much as the variants of a small grid differ by
-// (one launch of 14 us a run chose another plan from process to process).
+// (one launch of 14 us a run chose another plan from process to process).  The first
+// call on a grid pays for it, once in a process: over the passes of a damped tilt
+// series 11 ms at 256^2, 13 at 512^2, 28 at 1024^2 (with runs of 0.2 ms, five rounds: 22,
+// 28 and 40; with single launches 5, 11 and 31).
 template <typename F>
 bool time_variants(cudaStream_t s, int nv, F launch, float *ms)
 {
-    constexpr int kTuneRounds = 5;
-    constexpr float kTuneMs = 0.2f;
+    constexpr int kTuneRounds = 4;
+    constexpr float kTuneMs = 0.1f;
     std::vector<cudaEvent_t> ev((size_t)2 * nv * kTuneRounds, nullptr);
     bool ok = true;
     for (auto &e : ev) ok = ok && cudaEventCreate(&e) == cudaSuccess;
-    for (int w = 0; w < 2 && ok; w++)
-        for (int v = 0; v < nv; v++) launch(v);
+    for (int v = 0; v < nv && ok; v++) launch(v);
     int reps = 1;
     if (ok) {
         float t = 0.0f;
@@ -3811,8 +3813,9 @@ extern "C" int msk_tilt_series_batch(msk_context *ctx, const msk_series *s, int 
         }
         // the tuners run launches of their own: settle every choice first
         for (int i = first; i < last; i++) {
-            for (int mode : {(int)kColMask, (int)kColProp, (int)kColFresnel, (int)kColDW})
+            for (int mode : {(int)kColMask, (int)kColProp, (int)kColFresnel})
                 (void)col_variant(ctx, P[i].gp, mode);
+            if (!P[i].b.dw.empty()) (void)col_variant(ctx, P[i].gp, kColDW);
             (void)row_variant(ctx, P[i].gp);
         }
         cudaGraph_t gr = nullptr;
