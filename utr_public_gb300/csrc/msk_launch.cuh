@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <mutex>
 
+#include "device_once.h"
 #include "msk_passes.cuh"
 #include "msk_small.cuh"
 #include "msk_types.h"
@@ -20,13 +21,20 @@ struct ColView {
     int v;
 };
 
+inline int current_device()
+{
+    int d = -1;
+    return cudaGetDevice(&d) == cudaSuccess ? d : -1;
+}
+
 // SMs of the current device.
 inline int sm_count()
 {
     static std::mutex m;
     static int known[64];
-    int d = 0, n = 0;
-    if (cudaGetDevice(&d) != cudaSuccess || d < 0 || d >= 64) return 1;
+    const int d = current_device();
+    int n = 0;
+    if (d < 0 || d >= 64) return 1;
     std::lock_guard<std::mutex> lk(m);
     if (known[d]) return known[d];
     if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, d) != cudaSuccess || n < 1) return 1;
@@ -135,9 +143,9 @@ template <int N> struct Smem {
 };
 
 template <typename K>
-inline void set_smem(K kernel, size_t bytes, std::once_flag &flag)
+inline void set_smem(K kernel, size_t bytes, DeviceOnce &once)
 {
-    std::call_once(flag, [&] {
+    once.run(current_device(), [&] {
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
         // the default carve-out leaves ~100 KB of shared memory per SM, one
         // CTA of the larger passes; ask for the whole 228 KB
@@ -154,7 +162,7 @@ struct Launch {
     static void splat(const Geom &g, const int *units, int nunits, int slice, int nsl1,
                       const int *slice_off, const SplatAtom *atoms, float2 *tbuf, cudaStream_t s)
     {
-        static std::once_flag f;
+        static DeviceOnce f;
         set_smem(k_row_splat<N, kSplatTrans>, Smem<N>::splat, f);
         const int L = SplatCfg<N>::L;
         k_row_splat<N, kSplatTrans><<<nunits * row_blocks(g, L), L * P::T, Smem<N>::splat, s>>>(
@@ -164,7 +172,7 @@ struct Launch {
                                 const int *slice_off, const SplatAtom *atoms, float *vout,
                                 size_t vstride, cudaStream_t s)
     {
-        static std::once_flag f;
+        static DeviceOnce f;
         set_smem(k_row_splat<N, kSplatPot>, Smem<N>::splat, f);
         const int L = SplatCfg<N>::L;
         k_row_splat<N, kSplatPot><<<nunits * row_blocks(g, L), L * P::T, Smem<N>::splat, s>>>(
@@ -174,7 +182,7 @@ struct Launch {
                            const int *slice_off, const SplatAtom *atoms, float2 *spec,
                            cudaStream_t s)
     {
-        static std::once_flag f;
+        static DeviceOnce f;
         set_smem(k_row_splat<N, kSplatSpec>, Smem<N>::splat, f);
         const int L = SplatCfg<N>::L;
         k_row_splat<N, kSplatSpec><<<nunits * row_blocks(g, L), L * P::T, Smem<N>::splat, s>>>(
@@ -183,7 +191,7 @@ struct Launch {
     static void row_dwexp(const Geom &g, const int *units, int nunits, const float2 *spec,
                           float2 *tbuf, cudaStream_t s)
     {
-        static std::once_flag f;
+        static DeviceOnce f;
         set_smem(k_row_dwexp<N>, Smem<N>::row, f);
         const int L = RowCfg<N>::L;
         k_row_dwexp<N><<<nunits * row_blocks(g, L), L * P::T, Smem<N>::row, s>>>(g, units, spec,
@@ -195,7 +203,7 @@ struct Launch {
                      cudaStream_t s)
     {
         if (EV && !g.tw_col16) return;  // no table for the plan: nothing may run
-        static std::once_flag f;
+        static DeviceOnce f;
         constexpr size_t sm = Smem<N>::template col<V, EV>();
         set_smem(k_col_pass<N, MODE, V, EV>, sm, f);
         using CC = ColCfg<N, V, EV>;
@@ -254,7 +262,7 @@ struct Launch {
                                cudaStream_t s)
     {
         if (EV && !g.tw_row16) return;  // no 16-point twiddles bound: nothing to run
-        static std::once_flag f;
+        static DeviceOnce f;
         constexpr size_t sm = Smem<N>::template transmit<EV, W>();
         set_smem(k_row_transmit<N, SCAT, EV, W>, sm, f);
         constexpr int L = TrCfg<N, EV, W>::LT;
@@ -276,7 +284,7 @@ struct Launch {
             const int sms = sm_count();
             const long long njobs = (long long)nunits * (g.nx / R::RW);
             if (g.nx % R::RW || njobs < 5ll * sms * kRsWarps || njobs > 0x7fffffff) return false;
-            static std::once_flag fb, fw;
+            static DeviceOnce fb, fw;
             if (band && g.seg_e1 <= R::Z0 && g.seg_s2 >= R::Z1) {
                 set_smem(k_row_stream<N, SCAT, true>, R::SMEM, fb);
                 k_row_stream<N, SCAT, true><<<sms, 32 * kRsWarps, R::SMEM, s>>>(
@@ -311,7 +319,7 @@ struct Launch {
     static void row_init(const Geom &g, const int *units, int nunits, const float2 *wave0,
                          float2 *psi, float scale, cudaStream_t s)
     {
-        static std::once_flag f;
+        static DeviceOnce f;
         set_smem(k_row_simple<N, kRowInit>, Smem<N>::row, f);
         const int L = RowCfg<N>::L;
         k_row_simple<N, kRowInit><<<nunits * row_blocks(g, L), L * P::T, Smem<N>::row, s>>>(
@@ -320,7 +328,7 @@ struct Launch {
     static void row_band_inverse(const Geom &g, const int *units, int nunits, float2 *buf,
                                  cudaStream_t s)
     {
-        static std::once_flag f;
+        static DeviceOnce f;
         set_smem(k_row_simple<N, kRowBand>, Smem<N>::row, f);
         const int L = RowCfg<N>::L;
         k_row_simple<N, kRowBand><<<nunits * row_blocks(g, L), L * P::T, Smem<N>::row, s>>>(
@@ -329,7 +337,7 @@ struct Launch {
     static void row_inverse(const Geom &g, const int *units, int nunits, const float2 *in,
                             float2 *out, float scale, cudaStream_t s)
     {
-        static std::once_flag f;
+        static DeviceOnce f;
         set_smem(k_row_simple<N, kRowExit>, Smem<N>::row, f);
         const int L = RowCfg<N>::L;
         k_row_simple<N, kRowExit><<<nunits * row_blocks(g, L), L * P::T, Smem<N>::row, s>>>(
@@ -338,7 +346,7 @@ struct Launch {
     static void row_exit(const Geom &g, const int *units, int nunits, const float2 *psi,
                          float2 *out, cudaStream_t s)
     {
-        static std::once_flag f;
+        static DeviceOnce f;
         set_smem(k_row_simple<N, kRowExit>, Smem<N>::row, f);
         const int L = RowCfg<N>::L;
         k_row_simple<N, kRowExit><<<nunits * row_blocks(g, L), L * P::T, Smem<N>::row, s>>>(
@@ -349,7 +357,7 @@ struct Launch {
                                 const int *img_units, const int *img_dst, const int *img_flags,
                                 const float2 *ebuf, float *images, float nconf, cudaStream_t s)
     {
-        static std::once_flag f;
+        static DeviceOnce f;
         set_smem(k_row_intensity<N, SCAT>, Smem<N>::row, f);
         const int L = RowCfg<N>::L;
         k_row_intensity<N, SCAT><<<nimg * row_blocks(g, L), L * P::T, Smem<N>::row, s>>>(
@@ -359,7 +367,7 @@ struct Launch {
     static void row_expv(const Geom &g, int nunits, const float *v, size_t ustride, float2 *out,
                          cudaStream_t s)
     {
-        static std::once_flag f;
+        static DeviceOnce f;
         constexpr int L = RowCfg<N>::LT;
         constexpr size_t sm = (size_t)L * P::PADN * 8;
         set_smem(k_row_expv<N>, sm, f);
@@ -368,7 +376,7 @@ struct Launch {
     static void row_adj_transmit(const Geom &g, int nunits, float2 *Gu, float2 *B,
                                  const float2 *Wp, cudaStream_t s)
     {
-        static std::once_flag f;
+        static DeviceOnce f;
         set_smem(k_row_adj_transmit<N>, Smem<N>::adj, f);
         const int L = RowCfg<N>::LT;
         k_row_adj_transmit<N><<<nunits * row_blocks(g, L), L * P::T, Smem<N>::adj, s>>>(g, Gu, B, Wp);
@@ -376,7 +384,7 @@ struct Launch {
     static void row_grad(const Geom &g, int nunits, const float2 *Ge, const float *v,
                          size_t ustride, float *grad, cudaStream_t s)
     {
-        static std::once_flag f;
+        static DeviceOnce f;
         set_smem(k_row_grad<N>, Smem<N>::row, f);
         const int L = RowCfg<N>::L;
         k_row_grad<N><<<nunits * row_blocks(g, L), L * P::T, Smem<N>::row, s>>>(g, Ge, v, ustride,
@@ -385,7 +393,7 @@ struct Launch {
     static int row_imgrad(const Geom &g, int nunits, const float2 *E, const float *target,
                           size_t tstride, float2 *G, double *partial, cudaStream_t s)
     {
-        static std::once_flag f;
+        static DeviceOnce f;
         set_smem(k_row_imgrad<N>, Smem<N>::imgrad, f);
         const int L = RowCfg<N>::L;
         const int nb = nunits * row_blocks(g, L);
@@ -396,8 +404,8 @@ struct Launch {
     static cudaLaunchConfig_t small_cfg(int nunits, cudaStream_t s, cudaLaunchAttribute *at)
     {
         using C = SmallWaveCfg<N>;
-        static std::once_flag f;
-        std::call_once(f, [] {
+        static DeviceOnce f;
+        f.run(current_device(), [] {
             cudaFuncSetAttribute(k_small_wave<N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)C::SMEM);
             if (C::Q > 8)
@@ -487,7 +495,7 @@ struct Launch {
             if (device < 0 || device >= 64) return false;
             std::lock_guard<std::mutex> lk(m);
             if (!known[device]) {
-                static std::once_flag f;
+                static DeviceOnce f;
                 set_smem(k_wide_wave<N>, WideCfg<N>::SMEM, f);
                 int per = 0, coop = 0, sms = 0;
                 const bool ok =

@@ -38,7 +38,7 @@ template <int N> struct UtrLaunch {
     using P = FftPlan<N>;
     static void img_rows(const UtrImg &p, const float *img, float2 *k2, cudaStream_t s)
     {
-        static std::once_flag f;
+        static DeviceOnce f;
         set_smem(k_utr_img_rows<N>, Smem<N>::row, f);
         const int L = RowCfg<N>::L;
         k_utr_img_rows<N><<<(p.nrows + L - 1) / L, L * P::T, Smem<N>::row, s>>>(p, img, k2);
@@ -46,7 +46,7 @@ template <int N> struct UtrLaunch {
     static void fourier_rows(const UtrFourier &fr, const float2 *tw, const UtrAcc *acc,
                              float2 *vol, int nrows, cudaStream_t s)
     {
-        static std::once_flag f;
+        static DeviceOnce f;
         set_smem(k_utr_fourier_rows<N>, Smem<N>::row, f);
         const int L = RowCfg<N>::L;
         k_utr_fourier_rows<N><<<(nrows + L - 1) / L, L * P::T, Smem<N>::row, s>>>(fr, tw, acc, vol);
@@ -56,7 +56,7 @@ template <int N> struct UtrLaunch {
     {
         if constexpr (UtrTiltCfg<N>::OK) {
             using C = UtrTiltCfg<N>;
-            static std::once_flag f;
+            static DeviceOnce f;
             set_smem(k_utr_tilt_rows<N>, C::SMEM, f);
             const int kb = (p.nz + C::K - 1) / C::K;
             k_utr_tilt_rows<N><<<(unsigned)(p.ny * kb), C::NT, C::SMEM, s>>>(p, fr, tw16, vol);
@@ -66,7 +66,7 @@ template <int N> struct UtrLaunch {
     static void col(const UtrCol &p, const CUtensorMap &in, const CUtensorMap &out, int units,
                     cudaStream_t s)
     {
-        static std::once_flag f;
+        static DeviceOnce f;
         using CC = UtrColCfg<N, MODE == kUtrColFinal>;
         set_smem(k_utr_col<N, MODE>, CC::SMEM, f);
         const int bpu = p.ncb > 0 ? p.ncb : p.width / CC::C;
