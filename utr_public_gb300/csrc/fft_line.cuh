@@ -99,23 +99,31 @@ __host__ __device__ __forceinline__ float2 cfma(float m, float2 t, float2 u)
     return make_float2(fmaf(m, t.x, u.x), fmaf(m, t.y, u.y));
 #endif
 }
-__device__ __forceinline__ float2 cscale(float2 a, float s) { return up2(mul2(pk2(a.x, a.y), dup2(s))); }
+__host__ __device__ __forceinline__ float2 cscale(float2 a, float s)
+{
+#ifdef __CUDA_ARCH__
+    return up2(mul2(pk2(a.x, a.y), dup2(s)));
+#else
+    return make_float2(a.x * s, a.y * s);
+#endif
+}
 // The products' roundings are written out (two rounded products by b.y, then one
-// packed multiply-add by b.x), so that every kernel that runs the same transform --
+// multiply-add each by b.x), so that every kernel that runs the same transform --
 // a streamed and a plain form of a pass, one line or two at once -- gives the same
 // bits, whatever the compiler would contract.  The multipliers that carry a wave's
 // energy lie near 1 (transmissions, propagators of low frequencies): the products
 // by b.y are the small ones, and a part is rounded once at its full size.  With the
-// products by b.x rounded first it is rounded twice, for the same three
-// instructions (images against FP64: 1024^2, 160 slices 3.2e-6, now 2.9e-6; 512 x
-// 1024 2.5e-6, now 2.2e-6).
+// products by b.x rounded first it is rounded twice (images against FP64: 1024^2, 160
+// slices 3.2e-6, now 2.9e-6; 512 x 1024 2.5e-6, now 2.2e-6).  Both steps are packed:
+// 16 orientations of 1024^2 30.48 ms, one unit 4.17; with the products by b.y as two
+// scalar ones 30.69 and 4.20 (products by b.x first: 30.36 and 4.14).
 __host__ __device__ __forceinline__ float2 cmul(float2 a, float2 b)
 {
-    return cfma(b.x, a, make_float2(-(a.y * b.y), a.x * b.y));
+    return cfma(b.x, a, cscale(make_float2(-a.y, a.x), b.y));
 }
 __host__ __device__ __forceinline__ float2 cmul_conj(float2 a, float2 b)  // a * conj(b)
 {
-    return cfma(b.x, a, make_float2(a.y * b.y, -(a.x * b.y)));
+    return cfma(b.x, a, cscale(make_float2(a.y, -a.x), b.y));
 }
 
 __host__ __device__ constexpr int ilog2(int n)
