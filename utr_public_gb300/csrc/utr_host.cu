@@ -783,8 +783,9 @@ int msk_utr_reconstruct_planes(msk_context *ctx, const msk_utr *p, int nangles,
     // (5.4), from host images 10.1 (9.0), whose copy the general path's gridding
     // runs beside
     const UtrOps *xop = utr_ops(nx);
-    bool tilt = xop->tilt_rows && (size_t)ny * ((nz + xop->tilt_k - 1) / xop->tilt_k) >= 2 * 152 &&
-                2 * nz >= nx && std::isfinite(p->wl) && twiddles(nx, twx16, 16);
+    bool tilt = xop->tilt_rows && nz % xop->tilt_k == 0 &&
+                (size_t)ny * (nz / xop->tilt_k) >= 2 * (size_t)sm_count() && 2 * nz >= nx &&
+                std::isfinite(p->wl) && twiddles(nx, twx16, 16);
     for (int a = 0; a < nangles; a++) tilt = tilt && angles[2 * a] == 0.0 && std::isfinite(angles[2 * a + 1]);
     std::vector<float> tabs, scal, xs;
     grid_tables(p, g, nangles, tilt ? 1 : nangles, angles, tabs, scal, xs);

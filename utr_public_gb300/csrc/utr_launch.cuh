@@ -20,7 +20,7 @@ struct UtrOps {
                          int nrows, cudaStream_t);
     // gridding and fourier_rows in one pass, for orientations about y alone (tw16:
     // the 16-points-a-thread plan's twiddles); null for other lengths.  A CTA has
-    // tilt_k rows of consecutive z.
+    // tilt_k rows of consecutive z, and the depth is a multiple of that.
     int tilt_k;
     void (*tilt_rows)(const UtrGridP &, const UtrFourier &, const float2 *tw16, float2 *vol,
                       cudaStream_t);
@@ -58,8 +58,7 @@ template <int N> struct UtrLaunch {
             using C = UtrTiltCfg<N>;
             static DeviceOnce f;
             set_smem(k_utr_tilt_rows<N>, C::SMEM, f);
-            const int kb = (p.nz + C::K - 1) / C::K;
-            k_utr_tilt_rows<N><<<(unsigned)(p.ny * kb), C::NT, C::SMEM, s>>>(p, fr, tw16, vol);
+            k_utr_tilt_rows<N><<<(unsigned)(p.ny * (p.nz / C::K)), C::NT, C::SMEM, s>>>(p, fr, tw16, vol);
         }
     }
     template <int MODE>

@@ -340,11 +340,11 @@ k_utr_tilt_rows(const UtrGridP p, const UtrFourier f, const float2 *__restrict__
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     unsigned short *list = reinterpret_cast<unsigned short *>(smem + C::SUMS) + warp * SEG;
     UtrRow *rows = reinterpret_cast<UtrRow *>(smem + C::SUMS + (size_t)NW * SEG * 2);
-    const int kb = (p.nz + K - 1) / K;
+    const int kb = p.nz / K;  // whole blocks of rows (the dispatch's rule)
     const int J = blockIdx.x / kb, k0 = (blockIdx.x % kb) * K;
     float4 *z4 = reinterpret_cast<float4 *>(smem);
     for (int q = tid; q < K * S * 3 / 4; q += NT) z4[q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (tid < K) rows[tid] = utr_row(f, min(k0 + tid, p.nz - 1), J);
+    if (tid < K) rows[tid] = utr_row(f, k0 + tid, J);
     __syncthreads();
     const float xlo = p.fxlo, xhi = p.xs[NX - 1];
     for (int j = max(J - 1, 0); j <= min(J + 1, p.ny - 1); j++) {
@@ -499,11 +499,9 @@ k_utr_tilt_rows(const UtrGridP p, const UtrFourier f, const float2 *__restrict__
     for (int m = 0; m < E; m++) w[m] = make_float2(re[l * S + t + m * T], im[l * S + t + m * T]);
     __syncthreads();  // the exchange buffers lie over the sums
     fft_line<NX, false, 1, (T > 32), C::EV>(w, reinterpret_cast<float2 *>(smem) + l * C::P::PADN, 0, t, tw);
-    if (k < p.nz) {
-        float2 *dst = vol + ((size_t)k * p.ny + J) * NX;
+    float2 *dst = vol + ((size_t)k * p.ny + J) * NX;
 #pragma unroll
-        for (int m = 0; m < E; m++) dst[t + m * T] = w[m];
-    }
+    for (int m = 0; m < E; m++) dst[t + m * T] = w[m];
 }
 
 // ---------------------------------------------------------------- column passes
