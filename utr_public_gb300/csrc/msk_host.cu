@@ -1239,6 +1239,14 @@ int col_variant(msk_context *ctx, const GridPre &gp, int mode)
 // identically; the plans differ by FP32 rounding (another radix split of the
 // same transforms).  MSK_ROW_PLAN=0..2 in the environment fixes it.  The wave
 // and scattered forms share it.
+// One choice for calls of every size, so that a unit's bits do not depend on
+// how many run beside it; it is made on a launch of some tens of units (128 MB
+// of waves, 32 units at most), which streams (Launch::row_stream) at 1024^2 and
+// not on smaller square grids.  Smaller and larger calls than that, plan 0
+// (streamed when large) / plan 2 in ms: 1024^2 8 units 3.83 / 4.04, 16 units 7.2
+// / 7.7; 512^2 24 units 3.9 / 4.2, 90 units 8.8 / 9.7; 128^2 600 units 8.6 / 8.6;
+// but 256^2, where plan 2 is chosen, 45 units 3.16 / 3.06, 300 units 7.9 / 8.6:
+// a large series of 256^2 gains by MSK_ROW_PLAN=0.
 struct RowChoices {
     std::mutex m;
     std::map<std::array<int, 3>, int> v;  // (device, nx, ny) -> variant

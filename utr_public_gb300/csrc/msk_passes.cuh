@@ -146,10 +146,11 @@ template <int NY> struct RowCfg {
 };
 // The transmit's schedules, chosen per row length at run time by timing them
 // (the row tuner of the host code): the FFT plan EV and the CTA width W.
-//   variant 0: EV = 0 (32 points a thread); launches of enough rows of 64 to
-//              1024 points stream (k_row_stream), the others run in CTAs of 64
-//              threads (rows of up to 32 threads: two or more rows a CTA, so a
-//              CTA barrier waits for fewer warps; the registers of six CTAs per SM)
+//   variant 0: EV = 0 (32 points a thread); launches of at least five jobs of
+//              1024 points per warp of the GPU, rows of 64 to 1024 points,
+//              stream (k_row_stream), the others run in CTAs of 64 threads
+//              (rows of up to 32 threads: two or more rows a CTA, so a CTA
+//              barrier waits for fewer warps; the registers of six CTAs per SM)
 //   variant 1: EV = 0, CTAs of 128 threads (three per SM)
 //   variant 2: (64 to 2048 points) EV = 16 (16 points a thread), CTAs of 128
 //              threads, four per SM at 128 registers; a 2048-point row is one
