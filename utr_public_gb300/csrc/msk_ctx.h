@@ -73,8 +73,9 @@ enum Kind {
     kUtrImgRows, kUtrImgCols, kUtrGrid, kUtrFourier, kUtrVolCols, kUtrFinal, kUtrPoint,
     // the tilt series' image copy to host memory (event-timed, not a kernel)
     kCopyImages,
-    // the whole slice loop of a small grid in one cluster launch
-    kSmall,
+    // the wave chain of a group of slices in one launch (small grids, a lone unit), and
+    // the row pass that makes its transmissions iS(B)
+    kWaveChain, kBandInverse,
     kKinds
 };
 extern const char *const kKindName[kKinds];

@@ -1005,7 +1005,7 @@ const char *const kKindName[kKinds] = {
     "row_expv", "row_adj_transmit", "row_grad", "row_imgrad", "accumulate", "col_debye_waller",
     "row_dw_phase", "image_rotate_shift",
     "utr_image_rows", "utr_image_cols", "utr_grid", "utr_fourier_rows", "utr_volume_cols",
-    "utr_final_cols", "utr_pointwise", "copy_images_d2h", "small_slices"};
+    "utr_final_cols", "utr_pointwise", "copy_images_d2h", "wave_chain", "row_band_inverse"};
 }  // namespace msk
 
 namespace msk {
@@ -1840,7 +1840,7 @@ int run_slices(msk_context *ctx, const GridPre &gp, const Batch &b, int nmode, b
                               1.0f / ((float)gp.ny * (float)gp.ny), sA);
             }
             if (small || wide) {
-                Prof p(ctx, kExit, 16.0 * plane * na, sA);
+                Prof p(ctx, kBandInverse, 16.0 * plane * na, sA);
                 rop->row_band_inverse(g, grid_list, na, tb, sA);
             }
             if (overlap) {
@@ -1851,7 +1851,7 @@ int run_slices(msk_context *ctx, const GridPre &gp, const Batch &b, int nmode, b
         if (small || wide) {
             unsigned *count = reinterpret_cast<unsigned *>(ctx->flags.as<unsigned char>() + kWideCounter);
             if (wide) MSK_CUDA(ctx, cudaMemsetAsync(count, 0, sizeof(unsigned), sB));
-            Prof p(ctx, kSmall, plane * (24.0 * na + 16.0 * b.nunits * (s1 - s0)), sB);
+            Prof p(ctx, kWaveChain, plane * (24.0 * na + 16.0 * b.nunits * (s1 - s0)), sB);
             const int *so = ctx->slice_off.as<int>();
             const int arbitrary = w_in_band ? 0 : 1;
             MSK_CUDA(ctx, small ? cop->small_wave(g, b.nunits, s0, s1, nsl1, so, tb, psi, arbitrary, sB)
@@ -3455,12 +3455,12 @@ int enqueue_specimen(msk_context *ctx, SpecPlan &P, unsigned char *arena, const 
                 cop->col_mask(g, tmap, tmap, grid_list, nact, 1, 1.0f / ((float)ny * (float)ny), st);
             }
             if (P.small) {
-                Prof p(ctx, kExit, 16.0 * pl * nact, st);
+                Prof p(ctx, kBandInverse, 16.0 * pl * nact, st);
                 rop->row_band_inverse(g, grid_list, nact, tb, st);
             }
         }
         if (P.small) {
-            Prof p(ctx, kSmall, pl * (24.0 * nact + 16.0 * na * (s1 - s0)), st);
+            Prof p(ctx, kWaveChain, pl * (24.0 * nact + 16.0 * na * (s1 - s0)), st);
             MSK_CUDA(ctx, cop->small_wave(g, na, s0, s1, nsl1, soff, tb, psi, w_in_band ? 0 : 1, st));
             w_in_band = true;
             continue;

@@ -437,7 +437,8 @@ struct Launch {
             return cudaErrorNotSupported;
         }
     }
-    // clusters the device runs at once (cluster size and shared memory), 0 if none fit
+    // up to how many units the clusters beat the launch loop (SmallWaveCfg::PER CTAs
+    // an SM; with more they queue for SMs); 0 if the device fits no such cluster
     static int small_ok(int device)
     {
         if constexpr (N >= 64 && N <= 256) {
