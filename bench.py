@@ -662,7 +662,8 @@ def run_utr(args, rank, world, local_rank):
                                "volume of %.4g A voxels, CTF-3D + Ewald sphere correction, "
                                "aperture 40 mrad, NSR 0.03, epsilon 1e-4" % (n, n, FOV / n),
                    "voxels_per_step": nvox * world, "images_per_step": NANG * world,
-                   "l2": "inputs larger than L2 (34 GB of gridding sums per GPU)"},
+                   "l2": "inputs larger than L2 (image spectra and Fourier volume, %.1f GB per GPU)"
+                         % (8e-9 * (NANG * n * n + nvox))},
         "images_per_s": world * NANG / (ms / 1000.0),
         "e2e": {"value": world * nvox / (ms_e2e / 1000.0), "unit": UTR_UNIT,
                 "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(d2h),
